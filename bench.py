@@ -67,7 +67,7 @@ def parse():
     ap.add_argument("--k", type=int, default=0, help="inner dimension of the DGEMM extra (default: --size)")
     ap.add_argument("--no-extras", action="store_true", help="skip the DGEMM, grouped and CPU legs")
     ap.add_argument("--split-kernel", type=int, default=0, choices=(0, 1),
-                    help="real split kernel: 0 integer pipe (dp4a, default), 1 tensor core")
+                    help="real split kernel: 0 mma.sync (default), 1 tcgen05")
     ap.add_argument("--crt-kernel", type=int, default=2, choices=(0, 1, 2),
                     help="real CRT kernel: 2 auto (default: tensor core for 7- and 8-limb plans), 1 tensor core, 0 dp2a")
     ap.add_argument("--scale-fusion", type=int, default=0, choices=(0, 1),

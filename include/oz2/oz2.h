@@ -228,10 +228,11 @@ int oz2_set_failure_test(int64_t wait_limit_ns, int stall_mma);
 
 /* Kernel of the real split (no counterpart in the reference; process-wide, read when a call
  * builds its launches, so set it only while no other call is being made): 0 (default) the
- * integer-pipe (dp4a) split; 1 the tensor-core split, which computes the byte dot products of
+ * mma.sync split (byte dot products between registers); 1 the tcgen05 split, which computes those of
  * every residue with one tcgen05 u8 x u8 MMA per 512 elements (measured slower on B200: it is
- * bound by per-element instruction overhead, not by the dot products). Both write identical
- * planes. Complex operands always use the integer-pipe split. OZ2_EINVAL for other values. */
+ * bound by per-element instruction overhead, not by the dot products). Both write planes of the same
+ * residues modulo each m, so C is identical. Complex operands always use the mma.sync split.
+ * OZ2_EINVAL for other values. */
 int oz2_set_split_kernel(int kind);
 
 /* Kernel of the real CRT (no counterpart in the reference; process-wide, read when a call builds

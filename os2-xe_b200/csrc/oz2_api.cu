@@ -295,7 +295,7 @@ Sizes sizes_for(int64_t m, int64_t n, int64_t k, int s, int G, int64_t mb, int64
 }
 
 SplitItem side_item(const Prob& p, bool a_side, int64_t r0, int64_t rows, unsigned long long* maxbits,
-                    int8_t* planes, const ModConst* mc) {
+                    int8_t* planes) {
     SplitItem it{};
     const bool cplx = p.G == 3;
     const int w = cplx ? 2 : 1;
@@ -321,7 +321,7 @@ SplitItem side_item(const Prob& p, bool a_side, int64_t r0, int64_t rows, unsign
     it.planes = planes;
     it.kb_total = ceil_div(p.k, kTileK);
     it.plane_bytes = it.rows_pad * it.kb_total * kTileK;
-    for (int t = 0; t < it.s; ++t) it.mc[t] = mc[t];
+    for (int t = 0; t < it.s; ++t) it.mc[t] = p.plan->sm[t];
     return it;
 }
 
@@ -379,15 +379,14 @@ void plan_tasks(Program& prog, const std::vector<Task>& tasks, const GemmConfig&
     std::map<std::tuple<int, int, int>, std::vector<SplitItem>> split_groups;
     for (const Task& t : tasks) {
         const Prob& p = *t.p;
-        const ModConst* mc = p.plan->mc;
         const int wide = p.plan->tk > kWideScaleBits ? 2 : (p.plan->tk > kNarrowScaleBits ? 1 : 0);
         if (t.split_b) {
-            SplitItem it = side_item(p, false, t.j0, t.nb, t.maxB, t.planesB, mc);
+            SplitItem it = side_item(p, false, t.j0, t.nb, t.maxB, t.planesB);
             it.fuse = t.fuse_b;
             split_groups[{it.row_contig, it.cplx + 2 * it.fuse, wide}].push_back(it);
         }
         if (t.split_a) {
-            SplitItem it = side_item(p, true, t.i0, t.mb, t.maxA, t.planesA, mc);
+            SplitItem it = side_item(p, true, t.i0, t.mb, t.maxA, t.planesA);
             it.fuse = t.fuse_a;
             split_groups[{it.row_contig, it.cplx + 2 * it.fuse, wide}].push_back(it);
         }
@@ -2050,7 +2049,7 @@ int oz2_ozaki1_dgemm(oz2_handle h, int64_t m, int64_t n, int64_t k, const double
         Op op;
         op.kind = Op::Slice;
         op.count = 1;
-        op.blocks = split_item_blocks(it, 0);
+        op.blocks = slice_item_blocks(it, 0);
         op.off = prog.add(&it, sizeof it);
         prog.ops.push_back(op);
     }
@@ -2600,7 +2599,7 @@ int oz2_set_failure_test(int64_t wait_limit_ns, int stall_mma) {
 }
 
 int oz2_set_split_kernel(int kind) {
-    if (kind != 0 && kind != 1) return fail(nullptr, OZ2_EINVAL, "oz2: split kernel must be 0 (dp4a) or 1 (tensor core)");
+    if (kind != 0 && kind != 1) return fail(nullptr, OZ2_EINVAL, "oz2: split kernel must be 0 (mma.sync) or 1 (tensor core)");
     set_split_path(kind);
     return OZ2_OK;
 }

@@ -22,7 +22,8 @@ namespace oz2 {
 // A plane holds one modulus (and one 3M group) of one operand: rows x k int8 values stored as
 // row blocks of 128 rows, each made of k blocks of 128 bytes; one 128x128 tile is 16 KiB, row
 // r of the tile at r*128, 16-byte chunk c of that row at chunk position c ^ (r % 8). Rows and
-// k are zero-padded to whole tiles.
+// k are padded to whole tiles; k with zeros, rows with anything (no product of a padding row is
+// used).
 constexpr int kTileRows = 128;
 constexpr int kTileK = 128;
 constexpr int kTileBytes = kTileRows * kTileK;
@@ -75,7 +76,7 @@ struct SplitItem {
     int8_t* planes;                     // s planes (complex: 3 groups of s)
     int64_t plane_bytes, kb_total, rows_pad;
     int64_t block0, rblocks, kblocks;   // blocks = rblocks * kblocks
-    ModConst mc[kMaxModuliExt];
+    SplitMod mc[kMaxModuliExt];
     // tc: the tensor-core split runs this item (real operands); block0 is then its first unit of
     // 512 elements (4 rows x 128 inner indices, or 16 x 32 when rows are contiguous), rblocks x
     // kblocks its units
@@ -83,6 +84,8 @@ struct SplitItem {
     // fuse: the scale pass is fused into this item's split (real operands, k <= kFuseMaxK): the
     // kernel takes the row maxima itself and writes them to maxbits; rblocks blocks of whole rows
     int fuse;
+    int vec;    // 16-byte copies: every row (complex: every element) is 16-byte aligned
+    int kspan;  // k blocks of 128 inner indices per block of the launch
 };
 // largest k for which the scale pass is fused into the split (k contiguous / rows contiguous)
 constexpr int64_t kFuseMaxK = 2048;
@@ -145,11 +148,11 @@ struct CrtItem {
 
 // host-side helpers filling the launch-geometry fields; they return the blocks of the item
 int64_t scale_item_blocks(ScaleItem& it, int num_sms, int64_t block0);
-int64_t split_item_blocks(SplitItem& it, int64_t block0);
+int64_t slice_item_blocks(SplitItem& it, int64_t block0);
 // the split's geometry for the kernel that will run the item: the tensor-core split for real
 // items while it is selected, else split_item_blocks; sets it.tc
 int64_t split_geometry(SplitItem& it, int64_t block0);
-// process-wide selection of the real split: 0 the dp4a kernel (default), 1 the tensor-core split
+// process-wide selection of the real split: 0 the mma.sync kernel (default), 1 the tcgen05 split
 void set_split_path(int tc);
 int split_path();
 // process-wide: whether real operands with k <= kFuseMaxK (kFuseMaxKRowc when rows are contiguous)

@@ -155,14 +155,14 @@ extern "C" int oz2_dgemm_noalloc(void* stream, char ta, char tb, int64_t m, int6
     auto* planesB = reinterpret_cast<int8_t*>(scratch + o_B);
     unsigned char* resid = scratch + o_R;
     // the array keeps the previous call's contents: the error word and the maxima must start at
-    // zero; planes and residues are overwritten in full by the split and the first k chunk
+    // zero; planes and residues are overwritten by the split and the first k chunk (padding rows of
+    // the planes are not: no product of theirs is used)
     cudaError_t e = cudaMemsetAsync(scratch, 0, o_A, st);
     if (e != cudaSuccess) return reject(OZ2_ECUDA, std::string("oz2_dgemm_noalloc: ") + cudaGetErrorString(e));
 
     // item tables (one problem), written into the scratch by a kernel that takes them as its
     // parameter: host memory only, no staging buffer
-    ModConst mc[kMaxModuliExt];
-    mod_constants(p, mc);
+    const ModConst* mc = p.mc;
     struct Tables {
         ScaleItem sc[2];
         SplitItem sp[2];
@@ -194,7 +194,7 @@ extern "C" int oz2_dgemm_noalloc(void* stream, char ta, char tb, int64_t m, int6
         sp.plane_bytes = gg.plane_bytes;
         sp.kb_total = gg.kb_total;
         sp.rows_pad = gg.rows_pad;
-        for (int t = 0; t < s; ++t) sp.mc[t] = mc[t];
+        for (int t = 0; t < s; ++t) sp.mc[t] = p.sm[t];
         split_geometry(sp, 0);
     }
     GemmConfig cfg;

@@ -186,6 +186,7 @@ int make_plan_ext(int s, int64_t k, Plan& p) {
     if (tk > (s <= kMaxModuli ? kWideScaleBits : kMaxScaleBitsExt)) return 5;
     p = T.plan[s];
     p.tk = tk;
+    split_constants(p, p.sm);
     return 0;
 }
 
@@ -210,14 +211,10 @@ const char* plan_error_text(int s, int64_t k, int status, char* buf, int len) {
 
 void mod_constants(const Plan& p, ModConst* out) {
     for (int t = 0; t < p.s; ++t) {
-        const uint32_t m = p.m[t], h = (m - 1) / 2;
+        const uint32_t m = p.m[t];
         ModConst& c = out[t];
         c.m = m;
         c.mu = static_cast<uint32_t>((uint64_t{1} << 32) / m);
-        c.h = h;
-        c.koff3 = (h + m - pow2_mod(62, m)) % m;
-        c.koff5 = (h + m - pow2_mod(93, m)) % m;
-        c.koff7 = (h + m - pow2_mod(125, m)) % m;
         c.kbias = m * static_cast<uint32_t>(((uint64_t{1} << 31) + m - 1) / m);
         c.kbias30 = m * ((kExactSum + m - 1) / m);
         // Granlund and Montgomery (1994): with M = ceil(2^(32 + x) / m) = (2^(32 + x) + e) / m, e < m,
@@ -226,19 +223,23 @@ void mod_constants(const Plan& p, ModConst* out) {
         // with x = 7 and for m > 64 with x = 6
         c.mxs = m > 128 ? 7u : 6u;
         c.mx31 = static_cast<uint32_t>(((uint64_t{1} << (32 + c.mxs)) + m - 1) / m);
+    }
+}
+
+void split_constants(const Plan& p, SplitMod* out) {
+    const int words = split_words(p.tk), top = words == 2 ? 62 : (words == 3 ? 93 : 125);
+    for (int t = 0; t < p.s; ++t) {
+        const uint32_t m = p.m[t];
+        SplitMod& c = out[t];
         for (int w = 0; w < 4; ++w) {
             c.cb[w] = 0;
-            for (int b = 0; b < 4; ++b) c.cb[w] |= pow2_mod(8 * (4 * w + b), m) << (8 * b);
+            for (int b = 0; b < 4 && w < words; ++b) c.cb[w] |= pow2_mod(8 * (4 * w + b), m) << (8 * b);
         }
-        // division by a constant with an exact multiply-high (Granlund and Montgomery, 1994):
-        // with M = ceil(2^32 / m) = (2^32 + e) / m, 0 <= e < m <= 2^8, floor(v M / 2^32) =
-        // floor(v / m) for every v < 2^24 (the added v e / (m 2^32) stays below 1 / m)
-        c.m32 = static_cast<uint32_t>(((uint64_t{1} << 32) + m - 1) / m);
-        c.foff3 = 0x4B000000u + (m - pow2_mod(62, m)) % m;
-        c.foff5 = 0x4B000000u + (m - pow2_mod(93, m)) % m;
-        c.foff7 = 0x4B000000u + (m - pow2_mod(125, m)) % m;
+        c.m = m;
         c.finv = 1.0f / static_cast<float>(m);
-        c.fbias = -8388608.0f * c.finv;
+        c.off = (m - pow2_mod(top, m)) % m;
+        const uint32_t km = ((1u << 23) + m - 1) / m * m;
+        c.start = 0x4B000000u + (km - (1u << 23)) + c.off;
     }
 }
 

@@ -53,10 +53,6 @@ constexpr uint32_t kExactSum = 511u * 128u * 16384u;
 struct ModConst {
     uint32_t m;      // modulus
     uint32_t mu;     // floor(2^32 / m), Barrett
-    uint32_t h;      // (m - 1) / 2: residues are kept symmetric in [-h, m-1-h]
-    uint32_t koff3;  // (h - 2^62 mod m) mod m: narrow offset (tk <= 62)
-    uint32_t koff5;  // (h - 2^93 mod m) mod m: wide offset
-    uint32_t koff7;  // (h - 2^125 mod m) mod m: widest offset (extended plans)
     uint32_t kbias;  // m ceil(2^31 / m): c + kbias is in [0, 2^32) for every int32 GEMM sum c
                      // (|c| < 2^31 - 2^21) and congruent to c modulo m
     uint32_t kbias30;  // m ceil(kExactSum / m): c + kbias30 is in [0, 2^31) for every int32 GEMM sum
@@ -64,14 +60,22 @@ struct ModConst {
     uint32_t mx31;     // ceil(2^(32 + mxs) / m): floor(v / m) = umulhi(v, mx31) >> mxs exactly for v < 2^31
     uint32_t mxs;      // 7, or 6 for m < 128 (the moduli of the extended sets from s = 29), where
                        // ceil(2^39 / m) would not fit 32 bits
-    uint32_t cb[4];  // bytes 2^(8 l) mod m, l = 0..15, four per word (byte-limb weights)
-    uint32_t m32;    // ceil(2^32 / m): floor(v / m) = umulhi(v, m32) exactly for v < 2^24
-    // the split's start values 0x4B000000 + (-2^62 mod m), (-2^93 mod m), (-2^125 mod m): as
-    // floats, 2^23 plus the offset that cancels the narrow, wide and widest offset integers
-    uint32_t foff3, foff5, foff7;
-    float finv;   // fl(1 / m)
-    float fbias;  // -2^23 fl(1 / m), exact (a power-of-two multiple)
 };
+
+// Constants of one modulus as the split uses them, for the number of words of the plan's offset
+// integers (split_words). The byte dot product v = start + sum_l byte_l (2^(8 l) mod m) of an offset
+// integer x + 2^62 (2^93, 2^125) is the bit pattern of the float K m + v', with v' = off + sum_l ...
+// congruent to x and K m the first multiple of m from 2^23 on; one FMA by finv and 1.5 2^23 then
+// leaves K + rint(v' / m) in the low mantissa bits (oz2_split.cu: sym_residue).
+struct alignas(16) SplitMod {
+    uint32_t cb[4];  // bytes 2^(8 l) mod m, l = 0..15, four per word (byte-limb weights)
+    uint32_t m;
+    float finv;      // fl(1 / m)
+    uint32_t start;  // 0x4B000000 + (K m - 2^23) + off
+    uint32_t off;    // -2^62 (-2^93, -2^125) mod m
+};
+// 32-bit words of the offset integer of |x| <= 2^tk
+OZ2_HD constexpr int split_words(int tk) { return tk <= kNarrowScaleBits ? 2 : (tk <= kWideScaleBits ? 3 : 4); }
 
 struct Plan {
     int s = 0;
@@ -82,7 +86,8 @@ struct Plan {
     uint32_t y[kMaxModuliExt] = {};             // (M/m_t)^-1 mod m_t
     uint32_t W[kMaxModuliExt][kBigWords] = {};  // CRT weights (M/m_t) y_t
     uint32_t M[kBigWords] = {};
-    ModConst mc[kMaxModuliExt] = {};            // per-modulus kernel constants (mod_constants)
+    ModConst mc[kMaxModuliExt] = {};            // the GEMM's per-modulus constants (mod_constants)
+    SplitMod sm[kMaxModuliExt] = {};            // the split's (split_constants, for this tk)
 };
 
 // Returns 0, or 1 (invalid: s out of [2, 24], k < 1, s too small for k), or 5 (overflow).
@@ -95,6 +100,7 @@ int plan_tk(int s, int64_t k);
 const char* plan_error_text(int s, int64_t k, int status, char* buf, int len);
 
 void mod_constants(const Plan& p, ModConst* out);
+void split_constants(const Plan& p, SplitMod* out);
 
 // CRT table: Sum_t r_t W_t - q M with q = round(Sum_t r_t y_t / m_t) from an estimate whose
 // error is far below 1/4 (ref src/ozaki2_gpu.hpp:526-588 uses FP32; here 24-bit fixed point)

@@ -93,8 +93,8 @@ __device__ __forceinline__ double pow2(int k) {
 // |y| < 2^-1022, which rounds to 0 like the exact value), then one round-to-nearest-even
 // conversion. The offset integer 2^62 + x (narrow path, tk <= 62: x fits int64) as two 32-bit
 // words.
-__device__ __forceinline__ void offset_words_fp(double v, double s1, double s2, uint32_t (&W)[2]) {
-    const long long x = __double2ll_rn((v * s1) * s2);
+__device__ __forceinline__ void offset_words_fp(double y, uint32_t (&W)[2]) {
+    const long long x = __double2ll_rn(y);
     const uint64_t xo = static_cast<uint64_t>(x + (1ll << 62));
     W[0] = static_cast<uint32_t>(xo);
     W[1] = static_cast<uint32_t>(xo >> 32);
@@ -104,8 +104,8 @@ __device__ __forceinline__ void offset_words_fp(double v, double s1, double s2, 
 // <= 2^92 split exactly into hi = trunc(a 2^-64) and lo = a - hi 2^64 (both exact: power-of-two
 // scaling, and lo keeps a subset of a's 53 significant bits), then 2^93 +- (hi:lo), which lies in
 // (0, 2^94), as three 32-bit words.
-__device__ __forceinline__ void offset_words_fp_wide(double v, double s1, double s2, uint32_t (&W)[3]) {
-    const double y = rint((v * s1) * s2);
+__device__ __forceinline__ void offset_words_fp_wide(double y0, uint32_t (&W)[3]) {
+    const double y = rint(y0);
     const double a = fabs(y);
     const double hd = trunc(a * 5.421010862427522e-20);     // 2^-64
     const double ld = fma(hd, -18446744073709551616.0, a);  // a - hd 2^64, exact
@@ -126,8 +126,8 @@ __device__ __forceinline__ void offset_words_fp_wide(double v, double s1, double
 // Widest path (92 < tk <= 124, the extended moduli sets of the adaptive path): as the wide path
 // with a = |rint(y)| <= 2^124, hi = trunc(a 2^-64) < 2^60, and the offset 2^125 +- (hi:lo), which
 // lies in (0, 2^126), as four 32-bit words.
-__device__ __forceinline__ void offset_words_fp_widest(double v, double s1, double s2, uint32_t (&W)[4]) {
-    const double y = rint((v * s1) * s2);
+__device__ __forceinline__ void offset_words_fp_widest(double y0, uint32_t (&W)[4]) {
+    const double y = rint(y0);
     const double a = fabs(y);
     const double hd = trunc(a * 5.421010862427522e-20);     // 2^-64
     const double ld = fma(hd, -18446744073709551616.0, a);  // a - hd 2^64, exact
@@ -146,28 +146,25 @@ __device__ __forceinline__ void offset_words_fp_widest(double v, double s1, doub
     W[3] = static_cast<uint32_t>(oh >> 32);
 }
 
-// The byte dot products of the offset integer: v = 0x4B000000 + koff + sum_l byte_l (2^(8 l) mod m)
-// with koff = -2^62 (-2^93, -2^125) mod m, so that v' = v - 0x4B000000 is congruent to x modulo m
-// and below 2^20 (at most 16 bytes: m + 16 255^2), and v's bits are the float 2^23 + v' exactly.
-template <int NW>
-__device__ __forceinline__ uint32_t byte_dot(const uint32_t (&W)[NW], const ModConst& c) {
-    uint32_t v = NW == 2 ? c.foff3 : (NW == 3 ? c.foff5 : c.foff7);
-#pragma unroll
-    for (int j = 0; j < NW; ++j) v = __dp4a(W[j], c.cb[j], v);
-    return v;
-}
-
-// The symmetric residue v' - q m, q = rint(v' / m), in [-h, h] (m odd), in the low byte of the
-// result (the upper bytes hold a constant of m). One FMA gives fl(v' fl(1/m)): its addend -2^23
-// fl(1/m) cancels the 2^23 of v's float exactly, so only the product and one rounding err, by at
-// most (v'/m) 2^-23 < 2^-2 / m for v' < 2^21. For odd m, v'/m lies at least 1 / (2m) from every
-// half-integer, so adding 1.5 2^23 (round to nearest, ulp 1) gives the float 1.5 2^23 + q with
-// bits 0x4B400000 + q. Then v - bits m = v' - q m + (0x4B000000 - 0x4B400000 m), and both
-// constants are 0 modulo 256. Per residue: two FP32 operations in place of the integer
-// multiply-high quotient, and no shift of [0, m) to [-h, m-1-h] afterwards.
-__device__ __forceinline__ uint32_t sym_residue(uint32_t v, const ModConst& c) {
-    const float t = __fadd_rn(__fmaf_rn(__uint_as_float(v), c.finv, c.fbias), 12582912.0f);
-    return v - __float_as_uint(t) * c.m;
+// The symmetric residue v' - q m, q = rint(v' / m), in the low byte of the result (the upper bytes
+// hold anything), from the bits v of the float K m + v' (SplitMod). One FMA gives 1.5 2^23 + K + q
+// with a single rounding to an integer (ulp 1): the product errs by (K m + v') |fl(1/m) - 1/m| <
+// 0.63 / m, against a distance of at least 1 / (2 m) of v' / m from a half-integer (m odd), so q is
+// the nearest integer or, next to a tie, its neighbour: |residue| <= (m + 1) / 2 <= 127 for m <=
+// 253; fl(1/255) > 1/255, so m = 255 errs only upwards, to -128. Either way the byte is
+// congruent to x, which is all the INT8 products need (m = 256: any q gives the low byte of v').
+// v - bits m is v' - q m modulo 256: 0x4B000000, 2^22 and K m - K m are. Two instructions per residue.
+__device__ __forceinline__ uint32_t sym_residue(uint32_t v, float finv, uint32_t mneg) {
+    uint32_t r;  // in one piece: left to itself the compiler narrows the arithmetic to the byte it sees
+                 // used, which costs an instruction more per residue
+    asm("{\n\t.reg .f32 x, y;\n\t.reg .b32 t;\n\t"
+        "mov.b32 x, %1;\n\t"
+        "fma.rn.f32 y, x, %2, 0f4B400000;\n\t"  // + 1.5 2^23
+        "mov.b32 t, y;\n\t"
+        "mad.lo.u32 %0, t, %3, %1;\n\t}"
+        : "=r"(r)
+        : "r"(v), "f"(finv), "r"(mneg));
+    return r;
 }
 
 // low bytes of a, b, c, d as one little-endian word
@@ -175,193 +172,337 @@ __device__ __forceinline__ uint32_t pack_bytes(uint32_t a, uint32_t b, uint32_t 
     return __byte_perm(__byte_perm(a, b, 0x0040), __byte_perm(c, d, 0x0040), 0x5410);
 }
 
-// NLIMB: 3 selects the narrow path (two words per offset integer), 5 the wide one (three words),
-// 7 the widest (four words; real operands only: the complex path keeps s <= 24).
-// Elements per thread: 16 (one 16-byte chunk of every plane) on the real narrow path; 8 (half a
-// chunk) on the wide path (16 measured no faster) and for complex inputs (two groups of words)
-constexpr int kSplitRowcK = 256;  // inner indices per block of the rows-contiguous split
-
-template <int NLIMB, bool CPLX>
-__host__ __device__ constexpr int split_ept() {
-    return NLIMB == 3 && !CPLX ? 16 : 8;
+// D = C + A B: 16 x 32 by 32 x 8 unsigned bytes, int32 sums
+__device__ __forceinline__ void mma_u8(uint32_t (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1,
+                                       const uint4& c) {
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.u8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+        "{%10, %11, %12, %13};"
+        : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "r"(c.x), "r"(c.y), "r"(c.z), "r"(c.w));
+}
+__device__ __forceinline__ void mma_u8_add(uint32_t (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.u8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+        "{%0, %1, %2, %3};"
+        : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-// Each thread: one plane row r and EPT consecutive inner indices k0..k0+EPT-1 of every plane.
-// Block (bx, by) and thread -> plane row r and the first k0 of its EPT consecutive inner indices.
-// ROWC: a warp is EPT consecutive rows times 32 / EPT consecutive EPT-wide pieces: the loads along
-// r stay coalesced (EPT rows of 8 bytes per inner index), and the lanes of one row cover 32
-// inner indices, a whole 32-byte sector of each plane row (two 16-byte chunks that the swizzle
-// keeps adjacent); the 8 warps of a block continue along the inner index, so a block is EPT rows
-// by 256 inner indices. Otherwise a warp is one row and 32 consecutive pieces, the 8 warps are 8
-// rows.
-template <int EPT, bool ROWC>
-__device__ __forceinline__ void split_coords(int64_t bx, int64_t by, int64_t& r, int64_t& k0) {
-    const int lane = static_cast<int>(threadIdx.x & 31), warp = static_cast<int>(threadIdx.x >> 5);
-    if (ROWC) {
-        r = bx * EPT + lane % EPT;
-        k0 = by * kSplitRowcK + (warp * (32 / EPT) + lane / EPT) * EPT;
-    } else {
-        r = bx * 8 + warp;
-        k0 = by * (32 * EPT) + lane * EPT;
+template <int NW>
+__device__ __forceinline__ void offset_words(double y, uint32_t (&W)[NW]) {
+    if constexpr (NW == 2) offset_words_fp(y, W);
+    else if constexpr (NW == 3) offset_words_fp_wide(y, W);
+    else offset_words_fp_widest(y, W);
+}
+
+// The split's byte dot products run as mma.sync u8 x u8 -> s32 with the weights in A and the
+// offset integers in B, in a shape where no element leaves the lane that holds it: lane 4 n + q
+// gives column n of B the words of its own element in K positions q (bytes 4 q .. and 16 + 4 q ..),
+// and row (modulus t, q) of A (t < 4) holds modulus t's weights in K positions q and zeros
+// elsewhere, so entry ((t, q), n) of the product is the dot product of lane 4 n + q's element with
+// modulus t. One instruction gives 32 elements' residues for four moduli (two words; a second
+// instruction adds words 2 and 3), and lane (g, c) = (lane / 4, lane % 4) receives, for modulus
+// g % 4, those of the four lanes 4 n + q with n / 2 = c and q % 2 = g / 4. Every lane holds four
+// elements (j = 0..3) of a plane row's 128, lane 4 n + q the inner indices 16 ch + 4 j + sub with ch =
+// 2 (n / 2) + q % 2 and sub = n % 2 + 2 (q / 2): the sixteen residues that a lane receives from four
+// instructions are then the 16 bytes of one chunk of one plane, and a warp stores whole 128-byte
+// plane rows of four planes.
+//
+// Bound: instruction issue, then DRAM. A residue costs one FMA, one multiply-add, 3/4 of a byte
+// permute and 1/128 mma per lane (8.6 cycles of the scheduler per mma, measured) where dp4a took
+// two to four quarter-of-the-lanes dot products and a two-step quotient. The operand comes through
+// cp.async double buffering (rows contiguous: whole lines, transposed on the way out of shared
+// memory). Two blocks per SM of up to 128 registers on the narrow and complex paths, three of 80 on
+// the wider ones: more blocks with spilled or serialised accumulators measured slower. Stage times,
+// start -> now, alternating in one process: 8192^3 s = 16 1044 -> 682 us (498 us of DRAM time at the
+// measured copy rate), 6144^3 s = 20 (three words) 849 -> 575, 1024^2 x 262144 s = 16 3790 -> 2490,
+// ZGEMM 4096^3 s = 16 781 -> 424.
+constexpr int kSplitThreads = 256;
+constexpr int kSplitTileBytes = 16384;  // the operand's elements of one block tile
+// rows of a block tile (two per warp, one for complex operands), by 128 inner indices
+template <bool CPLX>
+__host__ __device__ constexpr int split_rows() { return CPLX ? 8 : 16; }
+
+// Shared memory of a block: two operand tiles, and the plan's constants per group of four moduli:
+// every lane's A fragments, the accumulators an mma starts from, and {-m, 1 / m, start - off} of the
+// lane's modulus (a group past s repeats modulus 0 and stores nothing).
+template <int NW>
+struct SplitShared {
+    alignas(128) unsigned char tile[2][kSplitTileBytes];
+    uint4 a[kMaxModuliExt / 4][NW > 2 ? 2 : 1][32];
+    uint4 start[kMaxModuliExt / 4][4];
+    uint4 c[kMaxModuliExt / 4][4];
+};
+template <int NW>
+__device__ __forceinline__ void split_consts(const SplitItem* __restrict__ I, SplitShared<NW>& S) {
+    const int lane = static_cast<int>(threadIdx.x & 31), g = lane >> 2, c = lane & 3, nmod = I->s;
+    for (int grp = static_cast<int>(threadIdx.x >> 5); 4 * grp < nmod; grp += kSplitThreads / 32) {
+        const int t = 4 * grp + (g & 3);
+        const SplitMod& sm = I->mc[t < nmod ? t : 0];
+        const uint32_t m0 = c == (g >> 2) ? 0xFFFFFFFFu : 0u, m1 = c == 2 + (g >> 2) ? 0xFFFFFFFFu : 0u;
+        S.a[grp][0][lane] = make_uint4(sm.cb[0] & m0, sm.cb[0] & m1, sm.cb[1] & m0, sm.cb[1] & m1);
+        if constexpr (NW > 2) S.a[grp][1][lane] = make_uint4(sm.cb[2] & m0, sm.cb[2] & m1, sm.cb[3] & m0, sm.cb[3] & m1);
+        if (lane < 16 && c == 0) {
+            S.start[grp][g] = make_uint4(sm.start, sm.start, sm.start, sm.start);
+            S.c[grp][g] = make_uint4(0u - sm.m, __float_as_uint(sm.finv), sm.start - sm.off, 0u);
+        }
     }
 }
 
-// The EPT elements (r, k0 .. k0 + EPT - 1) of every plane, r < rows_pad and k0 < the padded k:
-// maxb is the row's maximum bits (read only for r < rows).
-template <int NLIMB, bool CPLX, bool ROWC>
-__device__ __forceinline__ void split_piece(const SplitItem* __restrict__ I, int64_t r, int64_t k0,
-                                            unsigned long long maxb) {
-    constexpr int EPT = split_ept<NLIMB, CPLX>();
-    const int64_t kb_total = I->kb_total, plane_bytes = I->plane_bytes, ldx = I->ldx, k = I->k;
-    const int64_t rows = I->rows;
-    const double* X = I->X;
-    const int conj = I->conj, nmod = I->s;
-    const int64_t rb = r >> 7;
-    const int rr = static_cast<int>(r & 127);
-    const int64_t kb = k0 >> 7;
-    const int c = static_cast<int>((k0 >> 4) & 7);
-    int8_t* out = I->planes + (rb * kb_total + kb) * kTileBytes + rr * kTileK + ((c ^ (rr & 7)) << 4) +
-                  (k0 & 15);  // the second half of a chunk on the wide path
-    const int64_t gstride = static_cast<int64_t>(nmod) * plane_bytes;
-    auto store = [&](int8_t* dst, const uint32_t (&w)[EPT / 4]) {
-        if constexpr (EPT == 16) *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
-        else *reinterpret_cast<uint2*>(dst) = make_uint2(w[0], w[1]);
+// asynchronous copy of `bytes` (0: zeros) of 8 / 16 bytes to shared memory
+__device__ __forceinline__ void copy8(uint32_t dst, const void* src, int bytes) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void copy16(uint32_t dst, const void* src, int bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+
+// Where element (row r, inner index k) of a tile lies in shared memory, in elements. k contiguous:
+// [r][128]; rows contiguous: [k][rows]. The exclusive-or spreads the elements that the lanes of a
+// warp read together (inner indices 16 ch + 4 j + sub of one row, ch and sub by lane) over all banks
+// and keeps pairs of neighbours together.
+template <bool CPLX, bool ROWC>
+__device__ __forceinline__ int split_slot(int r, int k) {
+    if (ROWC) return k * split_rows<CPLX>() + (r ^ ((k & 3) | ((k >> 2) & (CPLX ? 4 : 12))));
+    return r * kTileK + (k ^ ((k >> 2) & (CPLX ? 4 : 12)));
+}
+
+// A thread's share of the copies of the block's tiles. k contiguous: warp w copies its own rows;
+// rows contiguous: the block copies whole lines. Tiles inside the operand take fixed strides from
+// one source and one shared-memory address; edge tiles check every element and read zeros outside.
+template <bool CPLX, bool ROWC>
+struct SplitFetch {
+    static constexpr int RB = split_rows<CPLX>(), E = CPLX ? 16 : 8;  // rows, bytes per element
+    static constexpr int R = RB / 8;
+    const char* src;  // of this thread's first element in the next tile
+    uint32_t dst;     // its shared-memory address in tile 0
+    int64_t step;     // source bytes between the thread's rows (k contiguous) or inner indices
+
+    __device__ __forceinline__ SplitFetch(const SplitItem* __restrict__ I, uint32_t tile0, int64_t r0, int kb0) {
+        const int tid = static_cast<int>(threadIdx.x), lane = tid & 31;
+        const int64_t ldx = I->ldx, k0 = static_cast<int64_t>(kb0) * kTileK;
+        int r, p;
+        if (ROWC) {
+            r = tid % RB, p = tid / RB;
+            step = ldx * (E * (kSplitThreads / RB));
+        } else {
+            r = R * (tid >> 5), p = lane * (I->vec ? 16 / E : 1);
+            step = ldx * E;
+        }
+        src = reinterpret_cast<const char*>(I->X) + (ROWC ? r0 + r + (k0 + p) * ldx : (r0 + r) * ldx + k0 + p) * E;
+        dst = tile0 + split_slot<CPLX, ROWC>(r, p) * E;
+    }
+
+    __device__ __forceinline__ void fast(uint32_t buf, bool vec) const {
+        const uint32_t d = dst + buf;
+        if (ROWC) {
+            const char* x = src;
+#pragma unroll
+            for (int i = 0; i < kTileK * RB / kSplitThreads; ++i, x += step) {
+                if (CPLX) {  // inner indices 32 apart: the same place in the swizzle
+                    const uint32_t to = d + i * (32 * RB * E);
+                    if (vec) {
+                        copy16(to, x, 16);
+                    } else {
+                        copy8(to, x, 8);
+                        copy8(to + 8, x + 8, 8);
+                    }
+                } else {  // inner indices 16 apart: swizzle bits 2, 3 of the row count them
+                    copy8((d ^ ((i & 3) << 5)) + i * (16 * RB * E), x, 8);
+                }
+            }
+        } else if (vec) {
+#pragma unroll
+            for (int u = 0; u < R; ++u) {
+                const char* x = u ? src + step : src;
+#pragma unroll
+                for (int i = 0; i < kTileK * E / 512; ++i) copy16(d + u * (kTileK * E) + 512 * i, x + 512 * i, 16);
+            }
+        } else {
+#pragma unroll
+            for (int u = 0; u < R; ++u) {
+                const char* x = u ? src + step : src;
+#pragma unroll
+                for (int i = 0; i < kTileK / 32; ++i) {
+                    if (CPLX) {
+                        copy8(d + 32 * E * i, x + 32 * E * i, 8);
+                        copy8(d + 32 * E * i + 8, x + 32 * E * i + 8, 8);
+                    } else {  // inner indices 32 apart: swizzle bit 3 alternates
+                        copy8((d ^ ((i & 1) << 6)) + u * (kTileK * E) + 32 * E * i, x + 32 * E * i, 8);
+                    }
+                }
+            }
+        }
+    }
+
+    // the tile at k0, with every access checked
+    __device__ __noinline__ static void edge(const SplitItem* __restrict__ I, uint32_t tile, int64_t r0, int k0) {
+        const int64_t rows = I->rows - r0, ldx = I->ldx;
+        const int k = static_cast<int>(I->k) - k0;
+        const char* X = reinterpret_cast<const char*>(I->X);
+        for (int f = static_cast<int>(threadIdx.x); f < kTileK * RB; f += kSplitThreads) {
+            // k contiguous: warp w takes its rows' elements, so that it alone waits for them
+            const int r = ROWC ? f % RB : R * static_cast<int>(threadIdx.x >> 5) + (f / kSplitThreads) * 32 / kTileK;
+            const int q = ROWC ? f / RB : (f / kSplitThreads * 32 + static_cast<int>(threadIdx.x & 31)) % kTileK;
+            const bool in = r < rows && q < k;
+            const char* x = in ? X + (ROWC ? r0 + r + (k0 + q) * ldx : (r0 + r) * ldx + k0 + q) * E : X;
+            const uint32_t to = tile + split_slot<CPLX, ROWC>(r, q) * E;
+            copy8(to, x, in ? 8 : 0);
+            if (CPLX) copy8(to + 8, x + 8, in ? 8 : 0);
+        }
+    }
+};
+
+// The block's rows r0 .. r0 + split_rows - 1 at the k blocks kb0 .. kb1 - 1: residues of the rows
+// below I->rows (the GEMM never uses a padding row's products) and of all inner indices (zero past
+// k). mx[r - mbase]: the rows' maximum bits. The next tile's copies run under this one's work.
+template <int NW, bool CPLX, bool ROWC>
+__device__ __forceinline__ void split_tiles(const SplitItem* __restrict__ I, SplitShared<NW>& S, int64_t r0, int kb0,
+                                            int kb1, const unsigned long long* mx, int64_t mbase) {
+    constexpr int R = split_rows<CPLX>() / 8, NG = CPLX ? 2 : 1, NP = CPLX ? 3 : 1, E = CPLX ? 16 : 8;
+    const int lane = static_cast<int>(threadIdx.x & 31), w8 = static_cast<int>(threadIdx.x >> 5);
+    const uint32_t tile0 = dev::smem_addr(S.tile[0]);
+    SplitFetch<CPLX, ROWC> F(I, tile0, r0, kb0);
+    const int64_t adv = ROWC ? I->ldx * (E * kTileK) : E * kTileK;
+    const bool vec = I->vec;
+    const int kfull = r0 + split_rows<CPLX>() <= I->rows ? static_cast<int>(I->k / kTileK) : 0;  // k blocks without edges
+    auto fetch = [&](int kb, uint32_t buf) {
+        if (kb < kfull) F.fast(buf, vec);
+        else SplitFetch<CPLX, ROWC>::edge(I, tile0 + buf, r0, kb * kTileK);
+        F.src += adv;
+        asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    if (r >= rows || k0 >= k) {  // padding: residues of zero are zero
-        const uint32_t z[EPT / 4] = {};
-        for (int t = 0; t < nmod; ++t) {
-            store(out + t * plane_bytes, z);
-            if (CPLX) {
-                store(out + gstride + t * plane_bytes, z);
-                store(out + 2 * gstride + t * plane_bytes, z);
-            }
-        }
-        return;
-    }
-    const int e = exponent_of(maxb, I->tk);
-    const bool live = e != kNonFinite;
-
-    constexpr int NG = CPLX ? 2 : 1;
-    constexpr int NW = NLIMB == 3 ? 2 : (NLIMB == 5 ? 3 : 4);  // 32-bit words of the offset integer
-    uint32_t L[NG][EPT][NW];
-    const int e1 = e >> 1;
-    const double s1 = pow2(live ? e1 : 0), s2 = pow2(live ? e - e1 : 0);
+    fetch(kb0, 0);
+    const int n = lane >> 2, q = lane & 3;
+    const int ch = 2 * (n >> 1) + (q & 1), sub = (n & 1) + 2 * (q >> 1);  // as a source of elements
+    const int64_t rw = r0 + R * w8;                                       // the warp's first row
+    const int64_t left = I->rows - rw;
+    const int nrows = left < R ? static_cast<int>(left) : R;
+    // scaling: 2^e in one exact factor; rows far up or down the exponent range take a second one,
+    // and a non-finite row's residues are zero (both rare, and the same for the whole warp)
+    double s1[R];
+    uint32_t odd = 0;
 #pragma unroll
-    for (int q = 0; q < EPT; ++q) {
-        const int64_t p = k0 + q;
-        double v0 = 0.0, v1 = 0.0;
-        if (live && p < k) {
-            const int64_t idx = ROWC ? r + p * ldx : p + r * ldx;
-            if (CPLX) {
-                v0 = __ldg(X + 2 * idx);
-                v1 = __ldg(X + 2 * idx + 1);
-                if (conj) v1 = -v1;  // residues of -y are the negated residues of y
-            } else {
-                v0 = __ldg(X + idx);
-            }
-        }
-        if constexpr (NLIMB == 3) {
-            offset_words_fp(v0, s1, s2, L[0][q]);
-            if (CPLX) offset_words_fp(v1, s1, s2, L[NG - 1][q]);
-        } else if constexpr (NLIMB == 5) {
-            offset_words_fp_wide(v0, s1, s2, L[0][q]);
-            if (CPLX) offset_words_fp_wide(v1, s1, s2, L[NG - 1][q]);
-        } else {
-            offset_words_fp_widest(v0, s1, s2, L[0][q]);
-        }
+    for (int u = 0; u < R; ++u) {
+        const int e = u < nrows ? exponent_of(mx[rw + u - mbase], I->tk) : 0;
+        const int e1 = max(-1000, min(1000, e));
+        s1[u] = pow2(e == kNonFinite ? 0 : e1);
+        if (e != e1) odd |= 1u << u;
     }
-
-    // real operands: two moduli per pass, so one modulus's constant loads and dot products overlap
-    // the other's (measured 2-12 % faster over the narrow, wide and widest paths; the complex path,
-    // whose registers are already high, measured slower with it)
-#pragma unroll(CPLX ? 1 : 2)
-    for (int t = 0; t < nmod; ++t) {
-        const ModConst mc = I->mc[t];
-        uint32_t b0[EPT], b1[EPT], b2[EPT];  // residue bytes in the low 8 bits
-        if (mc.m == 256) {
-            // 2^62 = 2^93 = 2^125 = 0 mod 256: the residue byte is the low byte of the offset integer
+    const double im_sign = CPLX && I->conj ? -1.0 : 1.0;  // residues of -y are the negated residues of y
+    // shared-memory address of the lane's element j = 0 of the warp's first row
+    const uint32_t el0 = tile0 + split_slot<CPLX, ROWC>(R * w8, 16 * ch + sub) * E;
+    // as a receiver: modulus g % 4 of each group of four, 16-byte chunk 2 c + g / 4 of the row
+    const int g = n, c = q, tl = g & 3, nmod = I->s;
+    const int64_t plane_bytes = I->plane_bytes, gstride = nmod * plane_bytes, tstep = 4 * plane_bytes;
+    const int rr = static_cast<int>(rw & 127), place = (2 * c + (g >> 2)) ^ (rr & 7);
+    int8_t* out0 = I->planes + ((rw >> 7) * I->kb_total + kb0) * kTileBytes + rr * kTileK + tl * plane_bytes + (place << 4);
+    const int next_row = kTileK + ((place & 1) ? -16 : 16);  // rr is even when a warp has two rows
+    for (int kb = kb0; kb < kb1; ++kb, out0 += kTileBytes) {
+        const uint32_t buf = ((kb - kb0) & 1) * kSplitTileBytes;
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        if (ROWC) __syncthreads();  // the whole block's copies; the other buffer's readers are done
+        else __syncwarp();
+        if (kb + 1 < kb1) fetch(kb + 1, buf ^ kSplitTileBytes);
+        if (nrows <= 0) continue;
+        uint32_t W[R][NG][4][NW];
 #pragma unroll
-            for (int q = 0; q < EPT; ++q) {
-                b0[q] = L[0][q][0];
-                if (CPLX) {
-                    b1[q] = L[NG - 1][q][0];
-                    b2[q] = b0[q] + b1[q];
+        for (int u = 0; u < R; ++u)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                // k contiguous: 4 j is bits 2, 3 of the inner index, which the swizzle flips
+                const uint32_t at = buf + (ROWC ? (el0 ^ (u * E)) + j * (4 * split_rows<CPLX>() * E)
+                                                : (CPLX ? (el0 ^ ((j & 1) << 6)) + ((j & 2) << 6) : (el0 ^ (j << 5))) +
+                                                      u * (kTileK * E));
+                double y[NG];
+                if (CPLX) asm("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(y[0]), "=d"(y[NG - 1]) : "r"(at));
+                else asm("ld.shared.f64 %0, [%1];" : "=d"(y[0]) : "r"(at));
+#pragma unroll
+                for (int h = 0; h < NG; ++h) {
+                    double x = y[h] * s1[u];
+                    if (CPLX && h) x *= im_sign;
+                    if (odd >> u & 1) {
+                        const int e = exponent_of(mx[rw + u - mbase], I->tk);
+                        x = e == kNonFinite ? 0.0 : x * pow2(e - max(-1000, min(1000, e)));
+                    }
+                    offset_words<NW>(x, W[u][h][j]);
                 }
             }
-        } else {
+        int8_t* out = out0;
+#pragma unroll 1
+        for (int grp = 0; 4 * grp < nmod; ++grp, out += tstep) {
+            const uint4 av = S.a[grp][0][lane], mc = S.c[grp][tl], start = S.start[grp][tl];
+            const uint32_t a[4] = {av.x, av.y, av.z, av.w};
+            uint32_t a2[4] = {};
+            if constexpr (NW > 2) {
+                const uint4 bv = S.a[grp][1][lane];
+                a2[0] = bv.x, a2[1] = bv.y, a2[2] = bv.z, a2[3] = bv.w;
+            }
+            const float finv = __uint_as_float(mc.y);
+            const bool valid = 4 * grp + tl < nmod;
 #pragma unroll
-            for (int q = 0; q < EPT; ++q) {
-                const uint32_t v0 = byte_dot<NW>(L[0][q], mc);
-                b0[q] = sym_residue(v0, mc);
-                if (CPLX) {
-                    const uint32_t v1 = byte_dot<NW>(L[NG - 1][q], mc);
-                    b1[q] = sym_residue(v1, mc);
-                    b2[q] = sym_residue(v0 + v1 - 0x4B000000u, mc);  // x0 + x1: v0' + v1' < 2^21
+            for (int u = 0; u < R; ++u) {
+                uint32_t w[NP][4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    uint32_t d[NG][4];
+#pragma unroll
+                    for (int h = 0; h < NG; ++h) {
+                        mma_u8(d[h], a, W[u][h][j][0], W[u][h][j][1], start);
+                        if constexpr (NW > 2) mma_u8_add(d[h], a2, W[u][h][j][2], NW > 3 ? W[u][h][j][NW - 1] : 0u);
+                    }
+#pragma unroll
+                    for (int h = 0; h < NP; ++h) {
+                        uint32_t r4[4];
+#pragma unroll
+                        for (int x = 0; x < 4; ++x)  // re + im: K m + (v0' + v1'), v0' + v1' < 2^21
+                            r4[x] = sym_residue(CPLX && h == 2 ? d[0][x] + d[NG - 1][x] - mc.z : d[h % NG][x], finv, mc.x);
+                        w[h][j] = pack_bytes(r4[0], r4[1], r4[2], r4[3]);
+                    }
+                }
+                if (valid && u < nrows) {
+                    int8_t* dst = out + u * next_row;
+#pragma unroll
+                    for (int h = 0; h < NP; ++h)
+                        *reinterpret_cast<uint4*>(dst + h * gstride) = make_uint4(w[h][0], w[h][1], w[h][2], w[h][3]);
                 }
             }
-        }
-        // the residue bytes (as int8), four per word
-        uint32_t w0[EPT / 4], w1[EPT / 4], w2[EPT / 4];
-#pragma unroll
-        for (int q = 0; q < EPT / 4; ++q) {
-            w0[q] = pack_bytes(b0[4 * q], b0[4 * q + 1], b0[4 * q + 2], b0[4 * q + 3]);
-            if (CPLX) {
-                w1[q] = pack_bytes(b1[4 * q], b1[4 * q + 1], b1[4 * q + 2], b1[4 * q + 3]);
-                w2[q] = pack_bytes(b2[4 * q], b2[4 * q + 1], b2[4 * q + 2], b2[4 * q + 3]);
-            }
-        }
-        store(out + t * plane_bytes, w0);
-        if (CPLX) {
-            store(out + gstride + t * plane_bytes, w1);
-            store(out + 2 * gstride + t * plane_bytes, w2);
         }
     }
 }
 
-template <int NLIMB, bool CPLX, bool ROWC>
-__device__ __forceinline__ void split_block(const SplitItem* __restrict__ items, int count) {
-    constexpr int EPT = split_ept<NLIMB, CPLX>();
+// A block: split_rows rows by I->kspan k blocks; block index -> (row block, k span)
+template <int NW, bool CPLX, bool ROWC>
+__global__ void __launch_bounds__(kSplitThreads, CPLX || NW == 2 ? 2 : 3)
+    split_kernel(const SplitItem* __restrict__ items, int count) {
+    __shared__ SplitShared<NW> S;
     const SplitItem* __restrict__ I = items + find_item(items, count, blockIdx.x);
     const int64_t local = static_cast<int64_t>(blockIdx.x) - I->block0;
     int64_t bx, by;
     divmod_index(local, I->rblocks, by, bx);
-    int64_t r, k0;
-    split_coords<EPT, ROWC>(bx, by, r, k0);
-    if (r >= I->rows_pad || k0 >= I->kb_total * kTileK) return;
-    split_piece<NLIMB, CPLX, ROWC>(I, r, k0, r < I->rows && k0 < I->k ? I->maxbits[r] : 0ull);
-}
-
-// Real operands: registers capped for three blocks of 256 per SM on the narrow path (16 elements
-// per thread, 80 registers) and four on the wide and widest paths (8 elements per thread, 64
-// registers, no spills). Complex operands keep the compiler's own allocation (two blocks per SM).
-template <int NLIMB, bool ROWC>
-__global__ void __launch_bounds__(256, NLIMB == 3 ? 3 : 4) split_kernel(const SplitItem* __restrict__ items, int count) {
-    split_block<NLIMB, false, ROWC>(items, count);
-}
-
-template <int NLIMB, bool ROWC>
-__global__ void __launch_bounds__(256) split_kernel_cplx(const SplitItem* __restrict__ items, int count) {
-    split_block<NLIMB, true, ROWC>(items, count);
+    split_consts<NW>(I, S);
+    __syncthreads();
+    const int kb0 = static_cast<int>(by) * I->kspan, kb1 = min(kb0 + I->kspan, static_cast<int>(I->kb_total));
+    split_tiles<NW, CPLX, ROWC>(I, S, bx * split_rows<CPLX>(), kb0, kb1, I->maxbits, 0);
 }
 
 // ------------------------------------------------------------------ scale fused into the split
 // One launch for both phases of a real operand (ref src/ozaki2_gpu.hpp:974-989 then :1004-1022
-// run them as two passes over A and B): a block owns whole plane rows, takes their maxima over
+// run them as two passes over A and B): a block owns RB whole plane rows, takes their maxima over
 // all of k (and writes them for the CRT), then splits the same rows. The second read of the rows
 // follows the first within the block, so it is served by L2 while the rows that all resident
 // blocks have in flight fit there (the launcher uses it for k up to kFuseMaxK: at most 8 rows of
-// 16 KiB, or 16 rows of 4 KiB, per block). k contiguous: 8 rows per block, a warp per row, lanes
-// over k. Rows contiguous: EPT rows per block (a 128-byte line per inner index), the 256 / EPT
-// thread groups over k, then the split's own warp layout over 256-wide k blocks.
-template <int NLIMB, bool ROWC>
-__global__ void __launch_bounds__(256) scale_split_kernel(const SplitItem* __restrict__ items, int count) {
-    constexpr int EPT = split_ept<NLIMB, false>();
-    constexpr int RB = ROWC ? EPT : 8;  // rows per block
+// 16 KiB, or 16 rows of 4 KiB, per block). k contiguous: a warp per row, lanes over k. Rows
+// contiguous: a line per inner index, the 256 / RB thread groups over k.
+template <int NW, bool ROWC>
+__global__ void __launch_bounds__(kSplitThreads) scale_split_kernel(const SplitItem* __restrict__ items, int count) {
+    constexpr int RB = split_rows<false>();  // rows per block
     __shared__ unsigned long long smax[RB];
+    __shared__ SplitShared<NW> S;
     const SplitItem* __restrict__ I = items + find_item(items, count, blockIdx.x);
+    split_consts<NW>(I, S);
     const int64_t r0 = (static_cast<int64_t>(blockIdx.x) - I->block0) * RB;
     const unsigned long long* X = reinterpret_cast<const unsigned long long*>(I->X);
-    const int64_t rows = I->rows, k = I->k, ldx = I->ldx, kpad = I->kb_total * kTileK;
+    const int64_t rows = I->rows, k = I->k, ldx = I->ldx;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid < RB) smax[tid] = 0;
     __syncthreads();
@@ -374,33 +515,25 @@ __global__ void __launch_bounds__(256) scale_split_kernel(const SplitItem* __res
         }
         if (best) atomicMax(&smax[tid % RB], best);
     } else {
-        const int64_t r = r0 + warp;
-        unsigned long long best = 0;
-        if (r < rows) {
+        for (int u = 0; u < RB / 8; ++u) {
+            const int64_t r = r0 + (RB / 8) * warp + u;
+            unsigned long long best = 0;
+            if (r < rows) {
 #pragma unroll 4
-            for (int64_t p = lane; p < k; p += 32) best = max(best, __ldg(X + p + r * ldx) & kAbsMask);
-        }
+                for (int64_t p = lane; p < k; p += 32) best = max(best, __ldg(X + p + r * ldx) & kAbsMask);
+            }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) best = max(best, __shfl_xor_sync(0xFFFFFFFFu, best, o));
-        if (lane == 0) smax[warp] = best;
+            for (int o = 16; o > 0; o >>= 1) best = max(best, __shfl_xor_sync(0xFFFFFFFFu, best, o));
+            if (lane == 0) smax[(RB / 8) * warp + u] = best;
+        }
     }
     __syncthreads();
     if (tid < RB && r0 + tid < rows) const_cast<unsigned long long*>(I->maxbits)[r0 + tid] = smax[tid];  // for the CRT
-    if (ROWC) {
-        for (int64_t by = 0; by * kSplitRowcK < kpad; ++by) {
-            int64_t r, k0;
-            split_coords<EPT, true>(blockIdx.x - I->block0, by, r, k0);  // bx: this block's EPT rows
-            if (r < I->rows_pad && k0 < kpad) split_piece<NLIMB, false, true>(I, r, k0, smax[r - r0]);
-        }
-    } else {
-        const int64_t r = r0 + warp;
-        if (r < I->rows_pad)
-            for (int64_t k0 = lane * EPT; k0 < kpad; k0 += 32 * EPT) split_piece<NLIMB, false, false>(I, r, k0, smax[warp]);
-    }
+    split_tiles<NW, false, ROWC>(I, S, r0, 0, static_cast<int>(I->kb_total), smax, r0);
 }
 
 // ------------------------------------------------------------------ tensor-core split
-// The byte dot products of byte_residue, v_t = Sum_l byte_l (2^(8 l) mod m_t), form a small
+// The byte dot products v_t = Sum_l byte_l (2^(8 l) mod m_t) form a small
 // matrix product: (moduli x bytes) times (bytes x elements). One tcgen05.mma kind::i8 (unsigned
 // A and B, M = 128, N = 256, K = 32, int32 in TMEM) computes them for a unit of 512 elements:
 //   B (N x K, K-major): column n holds two elements, segment g = 0, 1 in bytes 16 g .. 16 g + 15
@@ -413,7 +546,7 @@ __global__ void __launch_bounds__(256) scale_split_kernel(const SplitItem* __res
 // The epilogue turns v + koff into the residue (x + h) mod m by the exact multiply-high quotient
 // (v < 2^20), subtracts h modulo 256 and stores the 32 residues of one slot's 32 consecutive
 // inner indices as one 32-byte piece of its plane. The integer pipe keeps one multiply-high and
-// one multiply-subtract per residue; the dp4a of byte_residue move to the tensor core.
+// one multiply-subtract per residue.
 // Persistent, one CTA per SM with 16 warps, software-pipelined over the CTA's units: while the
 // MMA of unit k runs, the threads finish unit k - 1 from the other accumulator (two A and two B
 // tiles, 2 x 256 TMEM columns); a unit's FP64 loads are issued kTcAhead units ahead, into
@@ -457,17 +590,17 @@ struct TcGeom {
 };
 
 template <int NW>
-__device__ __forceinline__ void offset_words(double v, double s1, double s2, uint32_t (&W)[4]) {
+__device__ __forceinline__ void offset_words_padded(double y, uint32_t (&W)[4]) {
     if constexpr (NW == 2) {
         uint32_t w[2];
-        offset_words_fp(v, s1, s2, w);
+        offset_words_fp(y, w);
         W[0] = w[0], W[1] = w[1], W[2] = 0, W[3] = 0;
     } else if constexpr (NW == 3) {
         uint32_t w[3];
-        offset_words_fp_wide(v, s1, s2, w);
+        offset_words_fp_wide(y, w);
         W[0] = w[0], W[1] = w[1], W[2] = w[2], W[3] = 0;
     } else {
-        offset_words_fp_widest(v, s1, s2, W);
+        offset_words_fp_widest(y, W);
     }
 }
 
@@ -566,7 +699,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) split_tc_kernel(const SplitItem
                         const int sigma = 32 * ((tid >> 5) % q2) + (tid & 31);
                         uint4 w0 = make_uint4(0, 0, 0, 0), w1 = w0;
                         if (sigma < 2 * s) {
-                            const ModConst& c = I->mc[sigma % s];
+                            const SplitMod& c = I->mc[sigma % s];
                             const uint4 cw = make_uint4(c.cb[0], c.cb[1], NW > 2 ? c.cb[2] : 0u, NW > 3 ? c.cb[3] : 0u);
                             if (sigma < s) w0 = cw;
                             else w1 = cw;
@@ -581,7 +714,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) split_tc_kernel(const SplitItem
                 const int e1 = e >> 1;
                 const double s1 = pow2(live ? e1 : 0), s2 = pow2(live ? e - e1 : 0);
                 uint32_t W[4];
-                offset_words<NW>(pv[a], s1, s2, W);
+                offset_words_padded<NW>((pv[a] * s1) * s2, W);
                 *reinterpret_cast<uint4*>(sB0 + buf * 32768 + n_l * 128 + ((seg_l ^ (n_l & 7)) << 4)) =
                     make_uint4(W[0], W[1], W[2], W[3]);
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -620,12 +753,15 @@ __global__ void __launch_bounds__(kTcThreads, 1) split_tc_kernel(const SplitItem
                     valid = sigma < 2 * s;
                     if (valid) {
                         const int t = sigma % s;
-                        const ModConst& c = I->mc[t];
+                        const SplitMod& c = I->mc[t];
+                        const uint32_t h = (c.m - 1) / 2;  // residues symmetric in [-h, m - 1 - h]
                         seg = sigma / s;
                         m = c.m;
-                        m32 = c.m32;
-                        koff = NW == 2 ? c.koff3 : (NW == 3 ? c.koff5 : c.koff7);
-                        c256h = 256u - c.h;
+                        // ceil(2^32 / m): floor(v / m) = umulhi(v, m32) exactly for v < 2^24 (Granlund
+                        // and Montgomery, 1994)
+                        m32 = 0xFFFFFFFFu / m + 1u;
+                        koff = (h + c.off) % m;
+                        c256h = 256u - h;
                         plane = I->planes + t * I->plane_bytes;
                     }
                 }
@@ -707,16 +843,19 @@ __global__ void __launch_bounds__(kTcThreads, 1) split_tc_kernel(const SplitItem
 // Ozaki Scheme I digits (the reference's comparison baseline, benchmarks/ozaki1_gpu.hpp:31-40):
 // x = RNE(v 2^e) as on the narrow split path (tk = 7L - 2 <= 61), then L balanced base-128
 // digits in [-64, 63], most significant in plane 0, written in the same plane layout and with
-// the same thread mapping as split_kernel's narrow real path (16 elements per thread).
+// 16 elements of one row per thread. Rows contiguous: a warp is 16 rows by 2 pieces of 16 inner
+// indices, a block 16 rows by kSliceRowcK; otherwise a warp is one row by 32 pieces, a block 8 rows.
+constexpr int kSliceEpt = 16, kSliceRowcK = 256;
 template <bool ROWC>
 __global__ void __launch_bounds__(256) slice_kernel(const SplitItem* __restrict__ items, int count) {
-    constexpr int EPT = 16;
+    constexpr int EPT = kSliceEpt;
     const SplitItem* __restrict__ I = items + find_item(items, count, blockIdx.x);
     const int64_t local = static_cast<int64_t>(blockIdx.x) - I->block0;
     int64_t bx, by;
     divmod_index(local, I->rblocks, by, bx);
-    int64_t r, k0;
-    split_coords<EPT, ROWC>(bx, by, r, k0);
+    const int lane = static_cast<int>(threadIdx.x & 31), warp = static_cast<int>(threadIdx.x >> 5);
+    const int64_t r = ROWC ? bx * EPT + lane % EPT : bx * 8 + warp;
+    const int64_t k0 = ROWC ? by * kSliceRowcK + (warp * (32 / EPT) + lane / EPT) * EPT : by * (32 * EPT) + lane * EPT;
     const int64_t kb_total = I->kb_total, plane_bytes = I->plane_bytes, ldx = I->ldx, k = I->k;
     if (r >= I->rows_pad || k0 >= kb_total * kTileK) return;
     const int ndig = I->s;
@@ -772,21 +911,18 @@ void split_tc_dispatch(const SplitItem* d, int count, int64_t units, bool rowc, 
 std::atomic<int> g_split_tc{0};
 std::atomic<int> g_scale_fusion{0};
 
-template <int NLIMB>
+template <int NW>
 void scale_split_dispatch(const SplitItem* d, int count, int64_t blocks, bool rowc, cudaStream_t st) {
-    if (rowc) scale_split_kernel<NLIMB, true><<<static_cast<unsigned>(blocks), 256, 0, st>>>(d, count);
-    else scale_split_kernel<NLIMB, false><<<static_cast<unsigned>(blocks), 256, 0, st>>>(d, count);
+    const unsigned g = static_cast<unsigned>(blocks);
+    if (rowc) scale_split_kernel<NW, true><<<g, kSplitThreads, 0, st>>>(d, count);
+    else scale_split_kernel<NW, false><<<g, kSplitThreads, 0, st>>>(d, count);
 }
 
-template <int NLIMB, bool CPLX>
+template <int NW, bool CPLX>
 void split_dispatch(const SplitItem* d, int count, int64_t blocks, bool rowc, cudaStream_t st) {
-    if constexpr (CPLX) {
-        if (rowc) split_kernel_cplx<NLIMB, true><<<static_cast<unsigned>(blocks), 256, 0, st>>>(d, count);
-        else split_kernel_cplx<NLIMB, false><<<static_cast<unsigned>(blocks), 256, 0, st>>>(d, count);
-    } else {
-        if (rowc) split_kernel<NLIMB, true><<<static_cast<unsigned>(blocks), 256, 0, st>>>(d, count);
-        else split_kernel<NLIMB, false><<<static_cast<unsigned>(blocks), 256, 0, st>>>(d, count);
-    }
+    const unsigned g = static_cast<unsigned>(blocks);
+    if (rowc) split_kernel<NW, CPLX, true><<<g, kSplitThreads, 0, st>>>(d, count);
+    else split_kernel<NW, CPLX, false><<<g, kSplitThreads, 0, st>>>(d, count);
 }
 
 }  // namespace
@@ -813,36 +949,45 @@ int64_t scale_item_blocks(ScaleItem& it, int num_sms, int64_t block0) {
     return it.rblocks * ceil_div(it.k, it.kchunk);
 }
 
-int64_t split_item_blocks(SplitItem& it, int64_t block0) {
+int64_t slice_item_blocks(SplitItem& it, int64_t block0) {
     it.block0 = block0;
-    const int ept = it.tk > kNarrowScaleBits || it.cplx ? split_ept<5, false>() : split_ept<3, false>();
     const int64_t kpad = it.kb_total * kTileK;  // inner indices of the plane, padding included
     if (it.row_contig) {
-        it.rblocks = ceil_div(it.rows_pad, ept);
-        it.kblocks = ceil_div(kpad, kSplitRowcK);
+        it.rblocks = ceil_div(it.rows_pad, kSliceEpt);
+        it.kblocks = ceil_div(kpad, kSliceRowcK);
     } else {
         it.rblocks = ceil_div(it.rows_pad, 8);
-        it.kblocks = ceil_div(kpad, 32 * ept);
+        it.kblocks = ceil_div(kpad, 32 * kSliceEpt);
     }
     return it.rblocks * it.kblocks;
 }
 
 int64_t split_geometry(SplitItem& it, int64_t block0) {
+    it.block0 = block0;
+    const int rb = it.cplx ? split_rows<true>() : split_rows<false>();
+    // 16-byte copies where every row (every element of complex rows) is 16-byte aligned
+    it.vec = (reinterpret_cast<uintptr_t>(it.X) & 15) == 0 && (it.cplx || it.ldx % 2 == 0);
+    it.kspan = static_cast<int>(it.kb_total);
     if (it.fuse) {  // whole rows per block
         it.tc = 0;
-        it.block0 = block0;
-        const int rb = it.row_contig ? (it.tk > kNarrowScaleBits ? 8 : 16) : 8;
-        it.rblocks = it.rows_pad / rb;
+        it.rblocks = ceil_div(it.rows, rb);
         it.kblocks = 1;
         return it.rblocks;
     }
     it.tc = !it.cplx && g_split_tc.load() ? 1 : 0;
-    if (!it.tc) return split_item_blocks(it, block0);
-    it.block0 = block0;
-    const int ur = it.row_contig ? TcGeom<true>::UR : TcGeom<false>::UR;
-    const int uk = it.row_contig ? TcGeom<true>::UK : TcGeom<false>::UK;
-    it.rblocks = it.rows_pad / ur;              // rows_pad is a multiple of 128
-    it.kblocks = it.kb_total * (kTileK / uk);
+    if (it.tc) {
+        const int ur = it.row_contig ? TcGeom<true>::UR : TcGeom<false>::UR;
+        const int uk = it.row_contig ? TcGeom<true>::UK : TcGeom<false>::UK;
+        it.rblocks = it.rows_pad / ur;  // rows_pad is a multiple of 128
+        it.kblocks = it.kb_total * (kTileK / uk);
+        return it.rblocks * it.kblocks;
+    }
+    it.rblocks = ceil_div(it.rows, rb);
+    // up to 16 k blocks per block (a block's start costs about a tile's time: 8192^3 split 779, 697 and
+    // 682 us with at most 3, 8 and 16) while about four blocks per SM remain
+    const int64_t per = std::max<int64_t>(1, std::min<int64_t>(16, it.rblocks * it.kb_total / (4 * 148)));
+    it.kspan = static_cast<int>(per);
+    it.kblocks = ceil_div(it.kb_total, per);
     return it.rblocks * it.kblocks;
 }
 
@@ -888,29 +1033,23 @@ void launch_slice(const SplitItem* d, const SplitItem* h, int count, int64_t blo
 
 void launch_split(const SplitItem* d, const SplitItem* h, int count, int64_t blocks, int* err, cudaStream_t st) {
     if (count <= 0 || blocks <= 0) return;
-    const bool wide = h[0].tk > kNarrowScaleBits, rowc = h[0].row_contig != 0;
+    const int words = split_words(h[0].tk);
+    const bool rowc = h[0].row_contig != 0;
     if (h[0].fuse) {
-        if (h[0].tk > kWideScaleBits) scale_split_dispatch<7>(d, count, blocks, rowc, st);
-        else if (wide) scale_split_dispatch<5>(d, count, blocks, rowc, st);
-        else scale_split_dispatch<3>(d, count, blocks, rowc, st);
-        return;
-    }
-    if (h[0].tc) {
-        if (h[0].tk > kWideScaleBits) split_tc_dispatch<4>(d, count, blocks, rowc, err, st);
-        else if (wide) split_tc_dispatch<3>(d, count, blocks, rowc, err, st);
+        if (words == 4) scale_split_dispatch<4>(d, count, blocks, rowc, st);
+        else if (words == 3) scale_split_dispatch<3>(d, count, blocks, rowc, st);
+        else scale_split_dispatch<2>(d, count, blocks, rowc, st);
+    } else if (h[0].tc) {
+        if (words == 4) split_tc_dispatch<4>(d, count, blocks, rowc, err, st);
+        else if (words == 3) split_tc_dispatch<3>(d, count, blocks, rowc, err, st);
         else split_tc_dispatch<2>(d, count, blocks, rowc, err, st);
-        return;
-    }
-    if (h[0].tk > kWideScaleBits) {  // extended sets: real operands only
-        split_dispatch<7, false>(d, count, blocks, rowc, st);
-        return;
-    }
-    if (h[0].cplx) {
-        if (wide) split_dispatch<5, true>(d, count, blocks, rowc, st);
-        else split_dispatch<3, true>(d, count, blocks, rowc, st);
+    } else if (h[0].cplx) {  // s <= 24: at most three words
+        if (words == 3) split_dispatch<3, true>(d, count, blocks, rowc, st);
+        else split_dispatch<2, true>(d, count, blocks, rowc, st);
     } else {
-        if (wide) split_dispatch<5, false>(d, count, blocks, rowc, st);
-        else split_dispatch<3, false>(d, count, blocks, rowc, st);
+        if (words == 4) split_dispatch<4, false>(d, count, blocks, rowc, st);
+        else if (words == 3) split_dispatch<3, false>(d, count, blocks, rowc, st);
+        else split_dispatch<2, false>(d, count, blocks, rowc, st);
     }
 }
 

@@ -106,9 +106,9 @@ SPLIT_DEFAULT = SPLIT_DP4A
 
 
 def set_split_kernel(kind):
-    """Kernel of the real split (process-wide): SPLIT_DP4A (default, integer pipe) or
-    SPLIT_TENSOR_CORE (the residues' byte dot products as one tcgen05 u8 x u8 MMA per 512
-    elements; measured slower). Both write identical planes."""
+    """Kernel of the real split (process-wide): SPLIT_DP4A (default; the name is
+    historical: its byte dot products are mma.sync instructions) or SPLIT_TENSOR_CORE (the same as
+    one tcgen05 u8 x u8 MMA per 512 elements; measured slower). C is identical."""
     _raise(_lib.oz2_set_split_kernel(int(kind)))
 
 
