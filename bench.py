@@ -69,7 +69,7 @@ def parse():
     ap.add_argument("--split-kernel", type=int, default=0, choices=(0, 1),
                     help="real split kernel: 0 mma.sync (default), 1 tcgen05")
     ap.add_argument("--crt-kernel", type=int, default=2, choices=(0, 1, 2),
-                    help="real CRT kernel: 2 auto (default: tensor core for 7- and 8-limb plans), 1 tensor core, 0 dp2a")
+                    help="accepted for older command lines; there is one CRT kernel")
     ap.add_argument("--scale-fusion", type=int, default=0, choices=(0, 1),
                     help="scale pass fused into the split for k <= 2048 (1) or separate (0, default)")
     ap.add_argument("--crt-fusion", type=int, default=0, choices=(0, 1),

@@ -235,11 +235,8 @@ int oz2_set_failure_test(int64_t wait_limit_ns, int stall_mma);
  * OZ2_EINVAL for other values. */
 int oz2_set_split_kernel(int kind);
 
-/* Kernel of the real CRT (no counterpart in the reference; process-wide, read when a call builds
- * its launches): 0 the dp2a kernel; 1 the tensor-core CRT, whose limb sums are one tcgen05 u8 x
- * u8 MMA per 128 entries; 2 (default) the tensor-core CRT for plans of 7 and 8 limbs (s = 26..32),
- * the dp2a kernel below. All produce identical C. Complex operands always use the dp2a kernel. OZ2_EINVAL
- * for other values. */
+/* Kept for callers that chose between CRT kernels (0, 1 or 2; OZ2_EINVAL for other values): there is
+ * one CRT kernel, whose limb sums are mma.sync products, so every value has the same effect: none. */
 int oz2_set_crt_kernel(int kind);
 
 /* Scale pass fused into the split (no counterpart in the reference, which runs them as two passes

@@ -391,6 +391,7 @@ void plan_tasks(Program& prog, const std::vector<Task>& tasks, const GemmConfig&
             split_groups[{it.row_contig, it.cplx + 2 * it.fuse, wide}].push_back(it);
         }
     }
+    for (auto& kv : split_groups) split_launch_shape(kv.second.data(), static_cast<int>(kv.second.size()));
     for (auto& kv : split_groups) add_grouped(prog, kv.second, Op::Split, split_geom, nullptr, false);
     Op mk;
     mk.kind = Op::Mark;
@@ -507,11 +508,13 @@ void plan_tasks(Program& prog, const std::vector<Task>& tasks, const GemmConfig&
         c.br = p.beta[0];
         c.bi = p.beta[1];
         c.C = p.C + w * (t.i0 + t.j0 * p.ldc);
-        c.mma = crt_uses_mma(*p.plan, cplx) ? 1 : 0;
         auto& grp = crt_groups[{p.plan->s, cplx}];
         grp.first = p.plan;
         grp.second.push_back(c);
     }
+    for (auto& kv : crt_groups)
+        crt_launch_shape(kv.second.second.data(), static_cast<int>(kv.second.second.size()), *kv.second.first,
+                         kv.first.second != 0);
     for (auto& kv : crt_groups)
         add_grouped(prog, kv.second.second, Op::Crt, crt_geom, kv.second.first, kv.first.second != 0);
     mk.stage = kCrt;
@@ -669,8 +672,7 @@ void issue(oz2_context* h, const Program& prog, const unsigned char* dev) {
                                 h->d_err, h->stream);
                 break;
             case Op::Crt:
-                launch_crt(reinterpret_cast<const CrtItem*>(dev + op.off), op.count, op.blocks, *op.plan, op.cplx,
-                           h->d_err, h->stream);
+                launch_crt(reinterpret_cast<const CrtItem*>(dev + op.off), op.count, op.blocks, *op.plan, op.cplx, h->stream);
                 break;
             case Op::ScaleC: launch_scale_c(static_cast<double*>(op.ptr), op.ldc, op.m, op.n, op.beta, op.cplx, h->stream); break;
             case Op::Mark: mark(h, op.stage); break;
@@ -2605,8 +2607,7 @@ int oz2_set_split_kernel(int kind) {
 }
 
 int oz2_set_crt_kernel(int kind) {
-    if (kind < 0 || kind > 2) return fail(nullptr, OZ2_EINVAL, "oz2: CRT kernel must be 0 (dp2a), 1 (tensor core) or 2 (auto)");
-    set_crt_path(kind);
+    if (kind < 0 || kind > 2) return fail(nullptr, OZ2_EINVAL, "oz2: CRT kernel must be 0, 1 or 2");
     return OZ2_OK;
 }
 

@@ -1,5 +1,18 @@
 // oz2_crt_math.cuh - the exact CRT reconstruction of one C entry, shared by the CRT kernels
 // (oz2_crt.cu) and the GEMM whose epilogue runs the CRT for small s (oz2_gemm.cu).
+//
+// x = Sum_t r_t W_t - q M with q the nearest integer to Sum_t r_t W_t / M (|x| <= M/4), rounded once
+// to double. Everything runs on 16-bit limbs: a_l = Sum_t r_t W_t[l] as chains of two-way byte dot
+// products (dp2a; below 32 * 255 * 2^16 < 2^29), then
+//   q      from the top two limbs of the sum in FP32: the limbs below add less than 0.05 to Sum / M
+//          (0.03 for complex operands' signed sums), so the estimate errs by less than 1/4;
+//   limbs  c_l = a_l - q M_l + (c_{l-1} >> 16), one multiply-add and one shifted add each: the low 16
+//          bits of c_0 .. c_{L-2} and all of c_{L-1} are x in two's complement;
+//   RNE    the three top 32-bit words h, m, l as doubles (l with a sticky bit for the words below):
+//          h 2^32 + m rounds with an exact error term, and the last FMA rounds the exact sum once,
+//          signed numbers included. A top word that only repeats the sign is folded into the next.
+// The FP64 pipe takes over the sign, normalisation and rounding, which cost about 100 integer
+// instructions per entry as 64-bit words.
 #pragma once
 
 #include <cstdint>
@@ -16,136 +29,101 @@ __device__ __forceinline__ int exponent_of(unsigned long long b, int tk) {
     return tk - e2;
 }
 
-// 2^E * d for d in [2^63, 2^64]: exponent arithmetic on the bits while the result stays normal
-// (exact), ldexp otherwise (overflow, or one rounding into the subnormal range)
-__device__ __forceinline__ double scale_pow2(double d, int E) {
-    if (E >= -1022 - 63 && E <= 1023 - 64)
-        return __longlong_as_double(__double_as_longlong(d) + (static_cast<long long>(E) << 52));
-    return ldexp(d, E);
+// The exponent for the unscaling, with kFarExponent for a non-finite row or column: a sum of two
+// exponents (each within +-1200) at or above kFarExponent / 2 then means NaN.
+constexpr int kFarExponent = 1 << 20;
+__device__ __forceinline__ int unscale_exponent(unsigned long long b, int tk) {
+    const int e = exponent_of(b, tk);
+    return e == kNonFinite ? kFarExponent : e;
 }
 
-// Exact reconstruction + single rounding. R[g] holds the residues r_t in [0, m_t) of the moduli
-// 4g..4g+3 as bytes (zero past s). Every sum is a chain of two-way byte dot products (dp2a):
-// q = round(Sum r_t y_t / m_t) from the 16-bit fractions F16_t (error below 24 * 255 * 2^-16 <
-// 0.1, inside the 1/4 margin that |x| <= M/4 leaves, so q is the reference's FP32 quotient),
-// and Sum r_t W_t limb by limb over 16-bit limbs of W_t (each limb sum below 24 * 255 * 2^16 <
-// 2^29), then x = Sum r_t W_t - q M modulo 2^(32 NL) in 64-bit words, rounded once to double.
-template <int NL>
-__device__ __forceinline__ double crt_finish(const uint64_t (&acc)[NL], int64_t q, const uint32_t* Mw, int shift);
+// 32-bit words as doubles (exact)
+__device__ __forceinline__ double u32_double(uint32_t w) {
+    return __hiloint2double(0x43300000, static_cast<int>(w)) - 4503599627370496.0;  // 2^52
+}
+__device__ __forceinline__ double i32_double(int32_t w) {
+    return __hiloint2double(0x43300000, static_cast<int>(static_cast<uint32_t>(w) ^ 0x80000000u)) - 4503601774854144.0;  // 2^52 + 2^31
+}
 
-template <int S, int NL>
-__device__ __forceinline__ double crt_value(const uint32_t (&R)[(S + 3) / 4], const CrtConst& cc, int shift) {
-    constexpr int Q = (S + 3) / 4;
-    uint32_t uf = 1u << 15;  // rounding offset of the quotient
+// Limb l of the sums of EG entries: R[e][g] holds the residues (any byte congruent to r_t) of the
+// moduli 4g..4g+3 as bytes (zero past s); every weight word is read once for all entries.
+template <int Q, int EG>
+__device__ __forceinline__ void crt_limb(const uint32_t (&R)[EG][Q], const CrtConst& cc, int l, uint32_t (&a)[EG]) {
+#pragma unroll
+    for (int e = 0; e < EG; ++e) a[e] = 0;
 #pragma unroll
     for (int g = 0; g < Q; ++g) {
-        uf = __dp2a_lo(cc.Fq[g][0], R[g], uf);
-        uf = __dp2a_hi(cc.Fq[g][1], R[g], uf);
+        const uint32_t w0 = cc.Wq[g][l][0], w1 = cc.Wq[g][l][1];
+#pragma unroll
+        for (int e = 0; e < EG; ++e) a[e] = __dp2a_hi(w1, R[e][g], __dp2a_lo(w0, R[e][g], a[e]));
     }
-    const int64_t q = static_cast<int64_t>(uf >> 16);
-    uint64_t acc[NL];
+}
+
+// The 32-bit words of EG entries' x from the top: word k is the limbs L - 2 - 2k and L - 1 - 2k.
+// sum(l, a) gives limb l of the EG sums (signed for SIGNED); the top two come first, for the
+// quotient (the nearest integer to their part of the sum over M), the others as they are used.
+template <int L, int EG, bool SIGNED, class Sum>
+__device__ __forceinline__ void crt_words(Sum sum, const uint32_t* M16, const float* qf, uint32_t (&w)[EG][(L + 1) / 2]) {
+    uint32_t a1[EG], a0[EG], q[EG], c[EG];
+    sum(L - 1, a1);
+    if (L > 1) sum(L > 1 ? L - 2 : 0, a0);
 #pragma unroll
-    for (int l = 0; l < NL; ++l) {
-        uint32_t a0 = 0, a1 = 0;  // 16-bit limbs 2l and 2l + 1
+    for (int e = 0; e < EG; ++e) {
+        auto f = [](uint32_t v) { return SIGNED ? __int2float_rn(static_cast<int>(v)) : __uint2float_rn(v); };
+        float x = f(a1[e]) * qf[L - 1];
+        if (L > 1) x = __fmaf_rn(f(a0[e]), qf[L > 1 ? L - 2 : 0], x);
+        q[e] = __float_as_uint(__fadd_rn(x, 12582912.0f)) - 0x4B400000u;  // + 1.5 2^23
+    }
 #pragma unroll
-        for (int g = 0; g < Q; ++g) {
-            a0 = __dp2a_lo(cc.Wq[g][2 * l][0], R[g], a0);
-            a0 = __dp2a_hi(cc.Wq[g][2 * l][1], R[g], a0);
-            a1 = __dp2a_lo(cc.Wq[g][2 * l + 1][0], R[g], a1);
-            a1 = __dp2a_hi(cc.Wq[g][2 * l + 1][1], R[g], a1);
+    for (int l = 0; l < L; ++l) {
+        uint32_t a[EG];
+        if (l < L - 2) sum(l, a);
+#pragma unroll
+        for (int e = 0; e < EG; ++e) {
+            const uint32_t b = (l < L - 2 ? a[e] : (l == L - 2 ? a0[e] : a1[e])) - q[e] * M16[l];
+            const uint32_t prev = l ? c[e] : 0u;
+            c[e] = static_cast<uint32_t>(__dp2a_lo(static_cast<int>(prev), 0x100, static_cast<int>(b)));  // b + (prev >> 16)
+            if ((L - 1 - l) % 2 == 0) w[e][(L - 1 - l) / 2] = __byte_perm(prev, c[e], 0x5410);
         }
-        acc[l] = static_cast<uint64_t>(a0) + (static_cast<uint64_t>(a1) << 16);
     }
-    return crt_finish<NL>(acc, q, cc.M, shift);
 }
 
-// From the 32-bit limb sums acc[l] = sum_t r_t W_t[l] (below 2^46) and the quotient q: x = sum_t
-// r_t W_t - q M modulo 2^(32 NL) in 64-bit words (|x| <= M/4, two's complement), its magnitude's
-// leading 64 bits with a sticky bit for the rest, one RNE to double, 2^-shift.
-// The sums of crt_value for EG entries at once: every weight word is read once and used for all
-// of them (the entries' dot products interleave, and a constant costs one load, not EG). uf[e] is
-// the rounded quotient sum (q = uf >> 16) and acc[e][l] the limb sums of entry e.
-template <int S, int NL, int EG>
-__device__ __forceinline__ void crt_sums(const uint32_t (&R)[EG][(S + 3) / 4], const CrtConst& cc,
-                                         uint32_t (&uf)[EG], uint64_t (&acc)[EG][NL]) {
-    constexpr int Q = (S + 3) / 4;
+// x 2^-shift from x's words, rounded once (twice only into the subnormal range, as ldexp of the
+// rounded value); NaN when shift marks a non-finite row or column
+template <int L>
+__device__ __forceinline__ double crt_round(const uint32_t (&w)[(L + 1) / 2], int shift) {
+    constexpr int NW = (L + 1) / 2;
+    auto word = [&](int k) { return k < NW ? w[k < NW ? k : 0] : 0u; };
+    auto low = [&](int k) {  // word k with a sticky bit for the words below it
+        uint32_t rest = 0;
 #pragma unroll
-    for (int e = 0; e < EG; ++e) uf[e] = 1u << 15;
+        for (int i = 0; i < NW; ++i) rest |= i > k ? w[i] : 0u;
+        return word(k) | (rest != 0 ? 1u : 0u);
+    };
+    double dt = i32_double(static_cast<int32_t>(w[0]));
+    uint32_t m = word(1), l = low(2);
+    int E = 16 * L - 96 - shift;
+    if (w[0] + 1u <= 1u) {  // h is 0 or -1: x is small beside M
 #pragma unroll
-    for (int g = 0; g < Q; ++g) {
-        const uint32_t f0 = cc.Fq[g][0], f1 = cc.Fq[g][1];
-#pragma unroll
-        for (int e = 0; e < EG; ++e) uf[e] = __dp2a_hi(f1, R[e][g], __dp2a_lo(f0, R[e][g], uf[e]));
-    }
-#pragma unroll
-    for (int l = 0; l < NL; ++l) {
-        uint32_t a0[EG], a1[EG];  // 16-bit limbs 2l and 2l + 1
-#pragma unroll
-        for (int e = 0; e < EG; ++e) a0[e] = a1[e] = 0;
-#pragma unroll
-        for (int g = 0; g < Q; ++g) {
-            const uint32_t w00 = cc.Wq[g][2 * l][0], w01 = cc.Wq[g][2 * l][1];
-            const uint32_t w10 = cc.Wq[g][2 * l + 1][0], w11 = cc.Wq[g][2 * l + 1][1];
-#pragma unroll
-            for (int e = 0; e < EG; ++e) {
-                a0[e] = __dp2a_hi(w01, R[e][g], __dp2a_lo(w00, R[e][g], a0[e]));
-                a1[e] = __dp2a_hi(w11, R[e][g], __dp2a_lo(w10, R[e][g], a1[e]));
+        for (int k = 1; k < NW; ++k)
+            if (dt == 0.0 || dt == -1.0) {
+                dt = __fma_rn(dt, 4294967296.0, u32_double(w[k]));
+                m = word(k + 1);
+                l = low(k + 2);
+                E -= 32;
             }
-        }
-#pragma unroll
-        for (int e = 0; e < EG; ++e) acc[e][l] = static_cast<uint64_t>(a0[e]) + (static_cast<uint64_t>(a1[e]) << 16);
+        if (dt == 0.0) return shift >= kFarExponent / 2 ? __longlong_as_double(0x7FF8000000000000ll) : 0.0;
     }
-}
-
-template <int NL>
-__device__ __forceinline__ double crt_finish(const uint64_t (&acc)[NL], int64_t q, const uint32_t* Mw, int shift) {
-    // the quotient is below 2^16 (a 16-bit fraction sum shifted by 16), so q M_l is one
-    // 32 x 32 -> 64-bit product
-    const uint64_t q32 = static_cast<uint32_t>(q);
-    uint32_t w[NL];
-    int64_t carry = 0;
-#pragma unroll
-    for (int l = 0; l < NL; ++l) {
-        const int64_t v = static_cast<int64_t>(acc[l]) - static_cast<int64_t>(q32 * Mw[l]) + carry;
-        w[l] = static_cast<uint32_t>(v);
-        carry = v >> 32;
-    }
-    // 64-bit words, two's complement -> sign and magnitude
-    constexpr int NW = (NL + 1) / 2;
-    uint64_t X[NW];
-#pragma unroll
-    for (int i = 0; i < NW; ++i)
-        X[i] = static_cast<uint64_t>(w[2 * i]) | (2 * i + 1 < NL ? static_cast<uint64_t>(w[2 * i + 1]) << 32 : 0);
-    if (NL % 2)  // odd word count: sign-extend the top word into the last 64-bit word
-        X[NW - 1] = static_cast<uint64_t>(static_cast<int64_t>(static_cast<int32_t>(w[NL - 1])));
-    // magnitude without a branch: (X xor s) + (s & 1) over the words, s all ones when negative
-    const uint64_t sgn = static_cast<uint64_t>(static_cast<int64_t>(X[NW - 1]) >> 63);
-    uint64_t inc = sgn & 1u;
-#pragma unroll
-    for (int i = 0; i < NW; ++i) {
-        const uint64_t t = (X[i] ^ sgn) + inc;
-        inc &= t == 0 ? 1u : 0u;  // the carry goes on only past a word that wrapped to zero
-        X[i] = t;
-    }
-    // leading 64 bits with a sticky bit for everything below
-    uint64_t hiw = 0, low = 0;
-    bool sticky = false;
-    int tw = -1;
-#pragma unroll
-    for (int i = NW - 1; i >= 0; --i)
-        if (tw < 0 && X[i]) tw = i;
-    if (tw < 0) return 0.0;
-#pragma unroll
-    for (int i = 0; i < NW; ++i) {
-        if (i == tw) hiw = X[i];
-        else if (i == tw - 1) low = X[i];
-        else if (i < tw - 1) sticky |= X[i] != 0;
-    }
-    const int z = __clzll(static_cast<long long>(hiw));
-    const uint64_t top = z ? (hiw << z) | (low >> (64 - z)) : hiw;
-    sticky |= (z ? (low << z) : low) != 0;
-    const double val = scale_pow2(__ull2double_rn(top | (sticky ? 1u : 0u)), 64 * tw - z - shift);
-    return __longlong_as_double(__double_as_longlong(val) | static_cast<long long>(sgn & 0x8000000000000000ull));
+    // |dt| 2^32 > m, so the first sum's error is exact; (e 2^32 + l) is below 2^45 and exact; the
+    // sticky bit lies below half an ulp of the result, which is at least 2^64
+    const double s = __fma_rn(dt, 4294967296.0, u32_double(m));
+    const double e = u32_double(m) - __fma_rn(dt, -4294967296.0, s);
+    const double r = __fma_rn(s, 4294967296.0, __fma_rn(e, 4294967296.0, u32_double(l)));
+    // 2^64 <= |r| <= 2^98
+    if (static_cast<uint32_t>(E + 1086) <= 1086u + 924u)
+        return __hiloint2double(__double2hiint(r) + (E << 20), __double2loint(r));
+    if (shift >= kFarExponent / 2) return __longlong_as_double(0x7FF8000000000000ll);
+    return ldexp(r, E);
 }
 
 // 4 x 4 byte transpose: word t of `in` holds entries e = 0..3 of modulus 4g + t; word e of `out`

@@ -55,7 +55,8 @@ struct GemmParams {
     int* err;
     uint64_t wait_ns;  // limit of every bounded mbarrier wait
     int stall;         // failure-path test: the MMA issuer issues nothing, so the waits run out
-    CrtConst cc;       // kKindCrt: the plan's CRT constants (all items of the launch share the plan)
+    CrtConst cc;       // kKindCrt: the plan's CRT constants (all items of the launch share the plan),
+    int crt_shift;     // limbs moved up by this many bits to end at the fourth
 };
 
 struct Job {
@@ -365,8 +366,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_i8_modm_kernel(const __g
                             for (int q = 0; q < 8; ++q) {
                                 uint32_t r4[4];
 #pragma unroll
-                                for (int b = 0; b < 4; ++b) {
-                                    const uint32_t u = cur[4 * q + b] + kbias30;  // in [0, 2^31)
+                                for (int b = 0; b < 4; ++b) {  // byte 4 q + b: row q + 8 b of the 32
+                                    const uint32_t u = cur[q + 8 * b] + kbias30;  // in [0, 2^31)
                                     r4[b] = u - (__umulhi(u, mx31) >> mxs) * m;  // in [0, m)
                                 }
                                 w[q] = __byte_perm(__byte_perm(r4[0], r4[1], 0x0040),
@@ -389,7 +390,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_i8_modm_kernel(const __g
                             uint32_t r4[4];
 #pragma unroll
                             for (int b = 0; b < 4; ++b) {
-                                const uint32_t u = cur[4 * q + b] + kbias;  // c + m ceil(2^31/m), in [0, 2^32)
+                                const uint32_t u = cur[q + 8 * b] + kbias;  // c + m ceil(2^31/m), in [0, 2^32)
                                 uint32_t r = u - __umulhi(u, mu) * m;      // in [0, 2m)
                                 r = min(r, r - m);
                                 if (accumulate) {
@@ -419,7 +420,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_i8_modm_kernel(const __g
                     const int tk = I->crt_tk, s_ = I->s;
                     const int64_t j = static_cast<int64_t>(J.tj) * kGemmJ + quarter * 32 + lane;
                     const int64_t mm = I->m, nn = I->n;
-                    const int Ej = j < nn ? exponent_of(I->crt_maxB[j], tk) : 0;
+                    const int Ej = j < nn ? unscale_exponent(I->crt_maxB[j], tk) : 0;
                     const uint32_t rbase = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) +
                                            static_cast<uint32_t>(2 * BN + 128 * half);
 #pragma unroll 1
@@ -444,11 +445,13 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_i8_modm_kernel(const __g
                             for (int e = 0; e < 4; ++e) {
                                 const int64_t i = static_cast<int64_t>(J.ti) * BN + half * 64 + 4 * (8 * wb + q) + e;
                                 if (i < mm && j < nn) {
-                                    const int De = exponent_of(I->crt_maxA[i], tk);
-                                    const bool nonfinite = De == kNonFinite || Ej == kNonFinite;
-                                    const uint32_t R[2] = {lo[e], hi[e]};
-                                    double v = crt_value<kCrtFusedMaxS, 2>(R, P.cc, nonfinite ? 0 : De + Ej);
-                                    if (nonfinite) v = __longlong_as_double(0x7FF8000000000000ll);
+                                    const uint32_t R[1][2] = {{lo[e], hi[e]}};
+                                    // the launch's plan has L = one to four limbs: weights shifted up to the
+                                    // top of four (launch_gemm_crt), so that x comes out times 2^(16 (4 - L))
+                                    uint32_t xw[1][2];
+                                    crt_words<4, 1, false>([&](int l, uint32_t(&a)[1]) { crt_limb<2, 1>(R, P.cc, l, a); },
+                                                           P.cc.M16, P.cc.qf, xw);
+                                    const double v = crt_round<4>(xw[0], unscale_exponent(I->crt_maxA[i], tk) + Ej + P.crt_shift);
                                     double* cp = I->C + i + j * I->ldc;
                                     // the reference's unfused alpha*v + beta*c, one rounding per operation
                                     const double av = __dmul_rn(I->crt_alpha, v);
@@ -544,6 +547,14 @@ void launch_gemm_crt(const GemmItem* d_items, int count, int64_t jobs, const Pla
     if (count <= 0 || jobs <= 0) return;
     GemmParams P = make_params(d_items, count, group_j > 0 ? group_j : 16, jobs, err);
     crt_constants(plan, P.cc);
+    const int up = 4 - limbs16_for(plan.s);  // the kernel's CRT runs on four limbs
+    for (int l = 3; l >= 0; --l) {
+        for (int g = 0; g < 2; ++g)
+            for (int h = 0; h < 2; ++h) P.cc.Wq[g][l][h] = l >= up ? P.cc.Wq[g][l - up][h] : 0u;
+        P.cc.M16[l] = l >= up ? P.cc.M16[l - up] : 0u;
+        P.cc.qf[l] = l >= up ? P.cc.qf[l - up] : 0.0f;
+    }
+    P.crt_shift = 16 * up;
     const int grid = static_cast<int>(std::min<int64_t>(num_sms, jobs));
     launch_bn<128, kKindCrt>(P, grid, st);
 }

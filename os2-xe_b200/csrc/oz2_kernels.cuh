@@ -97,7 +97,7 @@ constexpr int kMaxOz1Pairs = 45;  // Ozaki Scheme I: L (L + 1) / 2 digit pairs, 
 struct GemmItem {
     const int8_t* planes_i;  // I side (op(A) rows), plane rows padded to 256
     const int8_t* planes_j;  // J side (op(B) columns), plane rows padded to 128
-    uint8_t* resid;          // residue planes [g][t]; entry (i, j) at (i / 32) * 32 n + j * 32 + i % 32
+    uint8_t* resid;          // residue planes [g][t]; entry (i, j) at (i / 32) * 32 n + j * 32 + 4 (i % 8) + i % 32 / 8
     int64_t pstride_i, pstride_j, rstride, ldr, m, n, kb_total;
     int64_t tiles, job0;
     int tiles_i, tiles_j, s, groups;
@@ -138,12 +138,8 @@ struct CrtItem {
     int tk;
     double ar, ai, br, bi;
     double* C;
-    int64_t block0, iblocks;  // blocks = ceil(n / jb) * iblocks
-    int tq, jb;               // a block: tq threads (4 rows each) along i x jb columns, tq * jb = 256
-    // mma: the tensor-core CRT (real items, crt_uses_mma): block0 is the first super-tile of 32
-    // rows x 16 columns (four tcgen05 MMAs of 128 entries) and iblocks the super-tiles along i;
-    // otherwise the dp2a kernel's geometry
-    int mma;
+    int64_t block0, iblocks;  // blocks = ceil(ceil(n / cols) / jc) * iblocks, iblocks = ceil(m / 32)
+    int cols, jc;             // a block: 32 rows x cols columns, jc times (crt_launch_shape)
 };
 
 // host-side helpers filling the launch-geometry fields; they return the blocks of the item
@@ -152,6 +148,8 @@ int64_t slice_item_blocks(SplitItem& it, int64_t block0);
 // the split's geometry for the kernel that will run the item: the tensor-core split for real
 // items while it is selected, else split_item_blocks; sets it.tc
 int64_t split_geometry(SplitItem& it, int64_t block0);
+// the k blocks per block of a split launch's items, before split_geometry
+void split_launch_shape(SplitItem* items, int count);
 // process-wide selection of the real split: 0 the mma.sync kernel (default), 1 the tcgen05 split
 void set_split_path(int tc);
 int split_path();
@@ -161,6 +159,8 @@ int split_path();
 // whether an operand qualifies
 void set_scale_fusion(int on);
 bool fuse_scale(bool cplx, bool row_contig, int64_t k);
+// sets the block shape of a CRT launch's items (all of one plan), before crt_item_blocks
+void crt_launch_shape(CrtItem* items, int count, const Plan& plan, bool cplx);
 int64_t crt_item_blocks(CrtItem& it, int64_t block0);
 
 // launches over device tables (d_items) whose host copies (h_items) give the geometry
@@ -202,21 +202,10 @@ void launch_oz1_horner(const int64_t* acc, int64_t m, int64_t n, int L, const un
                        const unsigned long long* maxB, int tk, double* C, int64_t ldc, cudaStream_t st);
 int64_t gemm_tiles_i(int64_t m, int bn);
 
-// whether launch_crt runs the tensor-core CRT for this plan (real items only): process-wide path
-// 0 the dp2a kernel, 1 the tensor-core CRT, 2 (default) the tensor-core CRT from
-// kCrtTcMinLimbs limbs on (7 and 8 limbs: s = 26..32, where it measured as fast or faster: B200,
-// 4096^2 x 1024, s = 29: 0.56 against 0.67 ms; s = 20: 0.47 against 0.28); the items' `mma` flag
-// must match
-constexpr int kCrtTcMinLimbs = 7;
-bool crt_uses_mma(const Plan& plan, bool cplx);
-void set_crt_path(int path);
-int crt_path();
-// sets the tensor-core CRT kernels' shared-memory attribute (with prepare_gemm_kernels)
+// sets the CRT kernels' shared-memory attribute (with prepare_gemm_kernels)
 cudaError_t prepare_crt_kernels();
-// all items of one CRT launch share s (the CRT table is a kernel parameter); err: the device error
-// word for the real kernel's bounded wait on its MMA (may be null)
-void launch_crt(const CrtItem* d_items, int count, int64_t blocks, const Plan& plan, bool cplx, int* err,
-                cudaStream_t st);
+// all items of one CRT launch share s (the CRT table is a kernel parameter)
+void launch_crt(const CrtItem* d_items, int count, int64_t blocks, const Plan& plan, bool cplx, cudaStream_t st);
 
 // sets the shared-memory attribute of the GEMM and tensor-core split kernels (once per device,
 // before any graph capture)

@@ -195,6 +195,7 @@ extern "C" int oz2_dgemm_noalloc(void* stream, char ta, char tb, int64_t m, int6
         sp.kb_total = gg.kb_total;
         sp.rows_pad = gg.rows_pad;
         for (int t = 0; t < s; ++t) sp.mc[t] = p.sm[t];
+        split_launch_shape(&sp, 1);
         split_geometry(sp, 0);
     }
     GemmConfig cfg;
@@ -238,7 +239,7 @@ extern "C" int oz2_dgemm_noalloc(void* stream, char ta, char tb, int64_t m, int6
     c.ar = alpha;
     c.br = beta;
     c.C = C;
-    c.mma = crt_uses_mma(p, false) ? 1 : 0;
+    crt_launch_shape(&c, 1, p, false);
     const int64_t crt_blocks = crt_item_blocks(c, 0);
     static_assert(sizeof(Tables) <= 8 * 1024, "item tables exceed their scratch region");
     unsigned char* dtab = scratch + o_D;
@@ -249,7 +250,7 @@ extern "C" int oz2_dgemm_noalloc(void* stream, char ta, char tb, int64_t m, int6
     for (int side = 1; side >= 0; --side)
         launch_split(&D->sp[side], &T.sp[side], 1, T.sp[side].rblocks * T.sp[side].kblocks, err, st);
     launch_gemm(&D->g, 1, g.tiles * s, cfg, num_sms, err, st);
-    launch_crt(&D->c, 1, crt_blocks, p, false, err, st);
+    launch_crt(&D->c, 1, crt_blocks, p, false, st);
     e = cudaGetLastError();
     return e == cudaSuccess ? OZ2_OK : reject(OZ2_ECUDA, std::string("oz2_dgemm_noalloc: ") + cudaGetErrorString(e));
 }

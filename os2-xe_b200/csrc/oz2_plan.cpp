@@ -120,7 +120,7 @@ struct Templates {
         p.log2M = M.log2();
         p.nl = static_cast<int>(std::floor(p.log2M / 32.0)) + 1;
         if (p.nl < 2) p.nl = 2;
-        if (p.nl != limbs_for(s)) return 3;
+        if (p.nl != limbs_for(s) || static_cast<int>(std::floor(p.log2M / 16.0)) + 1 != limbs16_for(s)) return 3;
         for (int t = 0; t < s; ++t) {
             Big Mt = M;
             if (Mt.divmod(p.m[t]) != 0) return 3;
@@ -131,6 +131,13 @@ struct Templates {
             p.y[t] = static_cast<uint32_t>(y);
         }
         std::memcpy(p.M, M.w, sizeof M.w);
+        // what the CRT's quotient leaves out, the limbs of Sum r_t W_t below the top two: under 0.1 M (two
+        // such sums for complex operands, s <= 24), inside the 1/4 that |x| <= M/4 leaves
+        double rest = 0.0;
+        for (int t = 0; t < s; ++t)
+            for (int l = 0; l < limbs16_for(s) - 2; ++l)
+                rest += 255.0 * std::exp2(16.0 * l - p.log2M) * ((p.W[t][l / 2] >> (16 * (l & 1))) & 0xFFFFu);
+        if (rest > 0.1) return 3;
         mod_constants(p, p.mc);
         return 0;
     }
@@ -243,20 +250,17 @@ void split_constants(const Plan& p, SplitMod* out) {
     }
 }
 
+uint32_t limb16(const uint32_t* w, int l) { return (w[l / 2] >> (16 * (l & 1))) & 0xFFFFu; }
+
 void crt_constants(const Plan& p, CrtConst& out) {
     out = CrtConst{};
-    out.s = p.s;
-    out.nl = p.nl;
-    for (int t = 0; t < p.s; ++t) {
-        const int g = t / 4, half = (t / 2) & 1, sh = 16 * (t & 1);
-        for (int l = 0; l < 2 * p.nl; ++l) {
-            const uint32_t w16 = (p.W[t][l / 2] >> (16 * (l & 1))) & 0xFFFFu;
-            out.Wq[g][l][half] |= w16 << sh;
-        }
-        const uint64_t f = ((static_cast<uint64_t>(p.y[t]) << 16) + p.m[t] / 2) / p.m[t];
-        out.Fq[g][half] |= static_cast<uint32_t>(std::min<uint64_t>(f, 0xFFFFu)) << sh;
+    double M = 0.0;
+    for (int i = p.nl - 1; i >= 0; --i) M = M * 4294967296.0 + p.M[i];
+    for (int l = 0; l < 2 * p.nl; ++l) {
+        for (int t = 0; t < p.s; ++t) out.Wq[t / 4][l][(t / 2) & 1] |= limb16(p.W[t], l) << (16 * (t & 1));
+        out.M16[l] = limb16(p.M, l);
+        out.qf[l] = static_cast<float>(std::ldexp(1.0, 16 * l) / M);
     }
-    for (int l = 0; l < p.nl; ++l) out.M[l] = p.M[l];
 }
 
 }  // namespace oz2

@@ -44,6 +44,13 @@ OZ2_HD constexpr int limbs_for(int s) {
     return t[s];
 }
 
+// 16-bit limbs of M per s: floor(log2 M / 16) + 1
+OZ2_HD constexpr int limbs16_for(int s) {
+    constexpr int t[kMaxModuliExt + 1] = {0, 0, 1,  2,  2,  3,  3,  4,  4,  5,  5,  6,  6,  7,  7,  8, 8,
+                                          9, 9, 10, 10, 11, 11, 12, 12, 12, 13, 13, 14, 14, 15, 15, 16};
+    return t[s];
+}
+
 // Constants of one modulus as the kernels use them.
 // GEMM sums of at most kExactKB k-blocks of 128 products of int8 residues are bounded by
 // kExactSum = 511 * 128 * 128^2 < 2^30, so c + kbias30 < 2^31 and the epilogue's quotient is exact
@@ -102,21 +109,18 @@ const char* plan_error_text(int s, int64_t k, int status, char* buf, int len);
 void mod_constants(const Plan& p, ModConst* out);
 void split_constants(const Plan& p, SplitMod* out);
 
-// CRT table: Sum_t r_t W_t - q M with q = round(Sum_t r_t y_t / m_t) from an estimate whose
-// error is far below 1/4 (ref src/ozaki2_gpu.hpp:526-588 uses FP32; here 24-bit fixed point)
+// CRT table: Sum_t r_t W_t - q M on 16-bit limbs, q from the sum's top two limbs in FP32 (the
+// reference estimates q from the residues in FP32, src/ozaki2_gpu.hpp:526-588)
 constexpr int kQuads = (kMaxModuliExt + 3) / 4;  // moduli in groups of four (one residue byte each)
+constexpr int kLimbs16 = 2 * kMaxLimbs;
 
 struct CrtConst {
-    int s, nl;
-    uint32_t M[kMaxLimbs];
     // W_t = (M / m_t) y_t in 16-bit limbs, paired for two-way byte dot products: for the moduli
     // 4g..4g+3 and limb l, Wq[g][l][0] = W16[4g][l] | W16[4g+1][l] << 16 and Wq[g][l][1] the same
     // for 4g+2, 4g+3 (zero past s)
-    uint32_t Wq[kQuads][2 * kMaxLimbs][2];
-    // F16_t = min(round(y_t / m_t 2^16), 2^16 - 1), paired the same way: fixed-point quotient
-    // weights (error per term below 2^-16, so for s <= 32 the quotient estimate is off by less than
-    // 1/8, inside the 1/4 margin that |x| <= M/4 leaves)
-    uint32_t Fq[kQuads][2];
+    uint32_t Wq[kQuads][kLimbs16][2];
+    uint32_t M16[kLimbs16];  // limbs of M
+    float qf[kLimbs16];      // 2^(16 l) / M (zero where it underflows)
 };
 void crt_constants(const Plan& p, CrtConst& out);
 

@@ -962,12 +962,21 @@ int64_t slice_item_blocks(SplitItem& it, int64_t block0) {
     return it.rblocks * it.kblocks;
 }
 
+void split_launch_shape(SplitItem* items, int count) {
+    // up to 16 k blocks per block (a block's start costs about a tile's time: 8192^3 split 779, 697 and
+    // 682 us with at most 3, 8 and 16) while about four blocks per SM remain in the launch
+    int64_t tiles = 0;
+    for (int q = 0; q < count; ++q)
+        tiles += ceil_div(items[q].rows, items[q].cplx ? split_rows<true>() : split_rows<false>()) * items[q].kb_total;
+    const int span = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(16, tiles / (4 * 148))));
+    for (int q = 0; q < count; ++q) items[q].kspan = span;
+}
+
 int64_t split_geometry(SplitItem& it, int64_t block0) {
     it.block0 = block0;
     const int rb = it.cplx ? split_rows<true>() : split_rows<false>();
     // 16-byte copies where every row (every element of complex rows) is 16-byte aligned
     it.vec = (reinterpret_cast<uintptr_t>(it.X) & 15) == 0 && (it.cplx || it.ldx % 2 == 0);
-    it.kspan = static_cast<int>(it.kb_total);
     if (it.fuse) {  // whole rows per block
         it.tc = 0;
         it.rblocks = ceil_div(it.rows, rb);
@@ -983,11 +992,7 @@ int64_t split_geometry(SplitItem& it, int64_t block0) {
         return it.rblocks * it.kblocks;
     }
     it.rblocks = ceil_div(it.rows, rb);
-    // up to 16 k blocks per block (a block's start costs about a tile's time: 8192^3 split 779, 697 and
-    // 682 us with at most 3, 8 and 16) while about four blocks per SM remain
-    const int64_t per = std::max<int64_t>(1, std::min<int64_t>(16, it.rblocks * it.kb_total / (4 * 148)));
-    it.kspan = static_cast<int>(per);
-    it.kblocks = ceil_div(it.kb_total, per);
+    it.kblocks = ceil_div(it.kb_total, it.kspan);
     return it.rblocks * it.kblocks;
 }
 

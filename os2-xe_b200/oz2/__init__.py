@@ -121,9 +121,8 @@ CRT_DEFAULT = CRT_AUTO
 
 
 def set_crt_kernel(kind):
-    """Kernel of the real CRT (process-wide): CRT_AUTO (default; the tensor-core CRT for 7- and
-    8-limb plans, s = 26..32, dp2a below), CRT_TENSOR_CORE (limb sums as one tcgen05 u8 x u8 MMA per 128
-    entries) or CRT_DP2A. All produce identical C."""
+    """Kept for callers that chose between CRT kernels: the three values are accepted and have no
+    effect (one kernel, whose limb sums are mma.sync products, measured faster for every plan)."""
     _raise(_lib.oz2_set_crt_kernel(int(kind)))
 
 
