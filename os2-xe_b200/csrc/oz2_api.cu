@@ -436,6 +436,7 @@ void plan_tasks(Program& prog, const std::vector<Task>& tasks, const GemmConfig&
         g.tiles = static_cast<int64_t>(g.tiles_i) * g.tiles_j;
         g.s = p.plan->s;
         g.groups = p.G;
+        g.f32 = f32_residues(*p.plan, g.kb_total) ? 1 : 0;
         g.job0 = jobs;
         const ModConst* mc = p.plan->mc;
         for (int q = 0; q < g.s; ++q) {
@@ -469,6 +470,7 @@ void plan_tasks(Program& prog, const std::vector<Task>& tasks, const GemmConfig&
         go.count = static_cast<int>(gi.size());
         go.jobs = jobs;
         go.cfg = cfg;
+        for (const GemmItem& g : gi) go.cfg.has_short |= g.f32 != 0;
         go.off = prog.add(gi.data(), gi.size() * sizeof(GemmItem));
         prog.ops.push_back(go);
     }
@@ -503,6 +505,7 @@ void plan_tasks(Program& prog, const std::vector<Task>& tasks, const GemmConfig&
         c.maxA = t.maxA + t.i0;
         c.maxB = t.maxB + t.j0;
         c.tk = p.plan->tk;
+        c.sgn = f32_residues(*p.plan, ceil_div(p.k, kTileK)) ? 1 : 0;
         c.ar = p.alpha[0];
         c.ai = p.alpha[1];
         c.br = p.beta[0];

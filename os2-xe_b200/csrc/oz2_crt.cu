@@ -1,5 +1,5 @@
-// oz2_crt.cu - CRT reconstruction of the Ozaki-II path: per C entry, s residues r_t in
-// [0, m_t) -> the exact integer x = Sum_t r_t W_t - q M (|x| <= M/4) -> one round-to-nearest-even to
+// oz2_crt.cu - CRT reconstruction of the Ozaki-II path: per C entry, s residues r_t
+// (bytes) -> the exact integer x = Sum_t r_t W_t - q M (|x| <= M/4) -> one round-to-nearest-even to
 // a double -> * 2^-(D_i + E_j) -> alpha/beta update (oz2_crt_math.cuh). Ref
 // src/ozaki2_gpu.hpp:526-588 (CrtAcc), :603-626 (launch_crt), :628-664 (launch_crt_cplx, 3M
 // recombination Re = P0 - P1, Im = P2 - P0 - P1).
@@ -9,6 +9,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cstring>
+#include <type_traits>
 
 #include "oz2_kernels.cuh"
 #include "oz2_crt_math.cuh"
@@ -19,7 +20,7 @@ namespace {
 
 // ---------------------------------------------------------------- CRT on mma.sync
 // The limb sums are a small integer matrix product, entries by moduli times moduli by weight bytes:
-// mma.sync u8 x u8 -> s32 with 16 entries in the rows of A, the moduli along K (16, or 32 for s > 16)
+// mma.sync u8 (signed residues: s8) x u8 -> s32 with 16 entries in the rows of A, the moduli along K (16, or 32 for s > 16)
 // and 8 bytes of W_t in the columns of B. A warp takes the 32 rows of a row block in one column at a
 // time: lane (g, c) = (lane / 4, lane % 4) reads the residue words (rows g, g + 8, g + 16, g + 24) of
 // the moduli 4 c .. 4 c + 3, and a 4 x 4 byte transpose makes them the A fragments of the four rows;
@@ -27,7 +28,7 @@ namespace {
 // the two bytes of one 16-bit limb, so it holds limb 4 T + c (tile T of 8 bytes) of four rows, which
 // go through shared memory to the lane of their row: lane l finishes row l (crt_words, crt_round)
 // and a warp reads and writes 32 consecutive entries of C. Complex: the three products' limb sums
-// are combined (Re = P0 - P1, Im = P2 - P0 - P1) before the quotient, which takes signed sums.
+// are combined (Re = P0 - P1, Im = P2 - P0 - P1) before the quotient.
 // Residues arrive through cp.async, four columns (one 128-byte line per plane) ahead.
 // Bound: instruction issue (166 warp instructions per 32 entries at s = 16, 34 cycles of them the four
 // mma at 8.6 each; the dp2a form it replaces took 304, 72 of them two-cycle dot products whose weights
@@ -54,16 +55,29 @@ struct CrtParams {
     alignas(16) uint8_t wb[2 * kLimbs16][32];  // byte b of W_t for t = 0..31 (zero past s)
 };
 
-__device__ __forceinline__ void mma_u8_k16(uint32_t (&d)[4], uint32_t a0, uint32_t a1, uint32_t b) {
-    asm("mma.sync.aligned.m16n8k16.row.col.s32.u8.u8.s32 {%0, %1, %2, %3}, {%4, %5}, {%6}, {%7, %7, %7, %7};"
-        : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
-        : "r"(a0), "r"(a1), "r"(b), "r"(0));
+// residues as signed or unsigned bytes times unsigned weight bytes
+template <bool SGN>
+__device__ __forceinline__ void mma_res_k16(uint32_t (&d)[4], uint32_t a0, uint32_t a1, uint32_t b) {
+    if constexpr (SGN)
+        asm("mma.sync.aligned.m16n8k16.row.col.s32.s8.u8.s32 {%0, %1, %2, %3}, {%4, %5}, {%6}, {%7, %7, %7, %7};"
+            : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
+            : "r"(a0), "r"(a1), "r"(b), "r"(0));
+    else
+        asm("mma.sync.aligned.m16n8k16.row.col.s32.u8.u8.s32 {%0, %1, %2, %3}, {%4, %5}, {%6}, {%7, %7, %7, %7};"
+            : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
+            : "r"(a0), "r"(a1), "r"(b), "r"(0));
 }
-__device__ __forceinline__ void mma_u8_k32(uint32_t (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
-                                           uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.u8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
-        : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0));
+template <bool SGN>
+__device__ __forceinline__ void mma_res_k32(uint32_t (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
+                                            uint32_t b0, uint32_t b1) {
+    if constexpr (SGN)
+        asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.u8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
+            : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
+            : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0));
+    else
+        asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.u8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
+            : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
+            : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0));
 }
 
 template <int L, bool CPLX>
@@ -91,7 +105,7 @@ __global__ void __launch_bounds__(256, CPLX ? 2 : (L <= 8 ? 4 : 3)) crt_kernel(c
     const int tk = I->tk, s = P.s;
     const int64_t m = I->m, n = I->n, ldc = I->ldc, i = ib * 32 + lane;
     const double ar = I->ar, ai = I->ai, br = I->br, bi = I->bi;
-    const bool beta = br != 0.0 || (CPLX && bi != 0.0), in = i < m;
+    const bool beta = br != 0.0 || (CPLX && bi != 0.0), in = i < m, sgn = I->sgn;
     const int De = in ? unscale_exponent(I->maxA[i], tk) : 0;
     const int64_t rstride = I->rstride, gstride = I->gstride;
     // the block's warps take neighbouring groups of COLS columns, I->jc times
@@ -163,32 +177,37 @@ __global__ void __launch_bounds__(256, CPLX ? 2 : (L <= 8 ? 4 : 3)) crt_kernel(c
                                            (COLS == 4 ? u * 128 : (u >> 1) * 128)));
                     transpose4(w[0], w[1], w[2], w[3], o[h][x]);
                 }
+            auto limbs = [&](auto sg) {
+                constexpr bool SGN = decltype(sg)::value;
 #pragma unroll
-            for (int T = 0; T < NT; ++T)
+                for (int T = 0; T < NT; ++T)
 #pragma unroll
-                for (int mt = 0; mt < 2; ++mt) {
-                    uint32_t v[G][2];
+                    for (int mt = 0; mt < 2; ++mt) {
+                        uint32_t v[G][2];
 #pragma unroll
-                    for (int h = 0; h < G; ++h) {
-                        uint32_t d[4];
-                        if constexpr (KH == 1) mma_u8_k16(d, o[h][0][2 * mt], o[h][0][2 * mt + 1], B[T][0]);
-                        else
-                            mma_u8_k32(d, o[h][0][2 * mt], o[h][0][2 * mt + 1], o[h][KH - 1][2 * mt],
-                                       o[h][KH - 1][2 * mt + 1], B[T][0], B[T][KH - 1]);
-                        v[h][0] = d[0] + (d[1] << 8);
-                        v[h][1] = d[2] + (d[3] << 8);
-                    }
+                        for (int h = 0; h < G; ++h) {
+                            uint32_t d[4];
+                            if constexpr (KH == 1) mma_res_k16<SGN>(d, o[h][0][2 * mt], o[h][0][2 * mt + 1], B[T][0]);
+                            else
+                                mma_res_k32<SGN>(d, o[h][0][2 * mt], o[h][0][2 * mt + 1], o[h][KH - 1][2 * mt],
+                                           o[h][KH - 1][2 * mt + 1], B[T][0], B[T][KH - 1]);
+                            v[h][0] = d[0] + (d[1] << 8);
+                            v[h][1] = d[2] + (d[3] << 8);
+                        }
 #pragma unroll
-                    for (int y = 0; y < 2; ++y) {
-                        const int row = 8 * (2 * mt + y) + g;
-                        if constexpr (CPLX) {  // |Re| < 2^29, |Im| < 2^30
-                            S.limb[0][row][4 * T + c] = v[0][y] - v[1][y];
-                            S.limb[CPLX][row][4 * T + c] = v[2 % G][y] - v[0][y] - v[1][y];
-                        } else {
-                            S.limb[0][row][4 * T + c] = v[0][y];
+                        for (int y = 0; y < 2; ++y) {
+                            const int row = 8 * (2 * mt + y) + g;
+                            if constexpr (CPLX) {  // below 2^31 in magnitude
+                                S.limb[0][row][4 * T + c] = v[0][y] - v[1][y];
+                                S.limb[CPLX][row][4 * T + c] = v[2 % G][y] - v[0][y] - v[1][y];
+                            } else {
+                                S.limb[0][row][4 * T + c] = v[0][y];
+                            }
                         }
                     }
-                }
+            };
+            if (sgn) limbs(std::true_type{});
+            else limbs(std::false_type{});
             __syncwarp();
             uint32_t a[CPLX ? 2 : 1][4 * NT];
 #pragma unroll
@@ -199,7 +218,7 @@ __global__ void __launch_bounds__(256, CPLX ? 2 : (L <= 8 ? 4 : 3)) crt_kernel(c
             __syncwarp();
             const int shift = De + __shfl_sync(0xFFFFFFFFu, Ec, k);
             uint32_t w[CPLX ? 2 : 1][(L + 1) / 2];
-            crt_words<L, CPLX ? 2 : 1, CPLX>(
+            crt_words<L, CPLX ? 2 : 1, true>(
                 [&](int l, uint32_t(&x)[CPLX ? 2 : 1]) {
                     x[0] = a[0][l];
                     if (CPLX) x[CPLX] = a[CPLX][l];

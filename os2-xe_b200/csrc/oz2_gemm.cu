@@ -14,15 +14,24 @@
 //            columns, double buffer); k beyond 130944 runs as chunks inside one job, each chunk
 //            adding its residues to the previous ones mod m
 //   warps 2-9 epilogue, two per TMEM lane quarter, each half of the BN columns: tcgen05.ld
-//            32 lanes x 32 columns (the next load in flight during the arithmetic), c mod m_t
-//            as (c + m ceil(2^31/m)) mod m with one Barrett step, 32 residue bytes per thread
-//            and chunk: a warp's 32 rows j x 32 columns i form one contiguous kilobyte of the
-//            residue plane (layout in oz2_kernels.cuh)
+//            32 lanes x 32 columns (the next load in flight during the arithmetic), the sum modulo
+//            m_t (at most 8 k-blocks: one FP32 FMA for the quotient, f32_residues; one exact chunk: a
+//            multiply-high quotient; else (c + m ceil(2^31/m)) mod m with one Barrett step), 32
+//            residue bytes per thread and chunk: a warp's 32 rows j x 32 columns i form one contiguous
+//            kilobyte of the residue plane (layout in oz2_kernels.cuh)
+// Bound: at long k the tensor pipe under the power limit (4096^3: 80 % active at 1.6 of 1.97 GHz); a pair
+// of CTAs per tile (cta_group::2, a third less L2 traffic) measured 4-10 % slower. At few k-blocks the
+// epilogue: B200, 6000^2 x 384, s = 16, 305 -> 255 us and 512 grouped problems 2577 -> 2037 us with the
+// FP32 quotient and items found by a cursor instead of a search per job and role.
 // Every mbarrier wait is time-bounded; on expiry the kernel records an error code, drains its
 // in-flight copies and MMAs, frees TMEM and returns.
 #include <algorithm>
 #include <atomic>
 #include <cstdio>
+#include <mutex>
+#include <set>
+
+#include <cuda.h>
 
 #include "oz2_crt_math.cuh"
 #include "oz2_kernels.cuh"
@@ -65,16 +74,32 @@ struct Job {
     int ti, tj;
     int64_t nch;  // k chunks
 };
-// per_tile: the job is a tile and runs every modulus (kKindCrt); otherwise (group, modulus, tile)
-__device__ __forceinline__ Job decode(const GemmParams& P, int64_t job, bool per_tile = false) {
-    int lo = 0, hi = P.count - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (P.items[mid].job0 <= job) lo = mid;
-        else hi = mid - 1;
+// The items of a role's increasing job numbers: one search for the first, then a step forward now
+// and then; the next item's first job is kept, so a job of the same item reads nothing.
+struct ItemCursor {
+    int item = 0;
+    int64_t next = -1;  // first job of item + 1 (-1: not searched yet)
+    __device__ __forceinline__ void find(const GemmItem* items, int count, int64_t job) {
+        if (next < 0) {
+            int hi = count - 1;
+            while (item < hi) {
+                const int mid = (item + hi + 1) >> 1;
+                if (items[mid].job0 <= job) item = mid;
+                else hi = mid - 1;
+            }
+        } else {
+            if (job < next) return;
+            ++item;
+            while (item + 1 < count && items[item + 1].job0 <= job) ++item;
+        }
+        next = item + 1 < count ? items[item + 1].job0 : INT64_MAX;
     }
+};
+// per_tile: the job is a tile and runs every modulus (kKindCrt); otherwise (group, modulus, tile)
+__device__ __forceinline__ Job decode(const GemmParams& P, ItemCursor& cur, int64_t job, bool per_tile = false) {
+    cur.find(P.items, P.count, job);
     Job J;
-    J.I = P.items + lo;
+    J.I = P.items + cur.item;
     // 32-bit arithmetic: an item's jobs (groups * s * tiles) are bounded by its residue planes,
     // s m n bytes of device memory, so they stay far below 2^32 (one 64-bit division costs
     // several times a 32-bit one, and every warp decodes every job)
@@ -104,7 +129,30 @@ __device__ __forceinline__ Job decode(const GemmParams& P, int64_t job, bool per
 // moduli: each modulus's residues go to tensor memory as packed bytes, columns 2 BN + 128 h + 16 t
 // + w for epilogue half h, modulus t and word w; after the last modulus the epilogue reconstructs
 // its 64 entries per lane and writes C)
-constexpr int kKindResidue = 0, kKindOz1 = 1, kKindCert = 2, kKindCrt = 3;
+// kKindShort as kKindResidue for launches with items of few k-blocks (GemmItem::f32), beside which others may
+// run; launches without them take the kernel without that code, which measured 0.5 % faster at long k
+constexpr int kKindResidue = 0, kKindOz1 = 1, kKindCert = 2, kKindCrt = 3, kKindShort = 4;
+
+// low bytes of a, b, c, d as one little-endian word
+__device__ __forceinline__ uint32_t pack_low(uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    return __byte_perm(__byte_perm(a, b, 0x0040), __byte_perm(c, d, 0x0040), 0x5410);
+}
+
+// The symmetric residue of an int32 sum |c| <= 2^24 in the low byte: q = rint(c fl(1/m)) with one rounding,
+// off by at most one where c / m is within 1 / m of a tie, so |c - q m| <= (m + 1) / 2 <= 127 for
+// m <= 253; below |c| = 2^23 the product errs by less than the 1 / (2 m) between c / m and a tie, and q is
+// exact for m = 255 as well. 1.5 2^23 leaves q in the low bits (0x4B400000 is 0 modulo 256).
+__device__ __forceinline__ uint32_t residue_f32(uint32_t c, float finv, uint32_t mneg) {
+    uint32_t r;  // in one piece: the compiler would narrow it to a byte, at an instruction more
+    asm("{\n\t.reg .f32 x, y;\n\t.reg .b32 t;\n\t"
+        "cvt.rn.f32.s32 x, %1;\n\t"
+        "fma.rn.f32 y, x, %2, 0f4B400000;\n\t"
+        "mov.b32 t, y;\n\t"
+        "mad.lo.u32 %0, t, %3, %1;\n\t}"
+        : "=r"(r)
+        : "r"(c), "f"(finv), "r"(mneg));
+    return r;
+}
 
 template <int BN, int KIND>
 __global__ void __launch_bounds__(kGemmThreads, 1) gemm_i8_modm_kernel(const __grid_constant__ GemmParams P) {
@@ -155,8 +203,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_i8_modm_kernel(const __g
             uint32_t phase = 0;
             uint32_t issued_mask = 0, issued_phase = 0;
             bool ok = true;
+            ItemCursor cursor;
             for (int64_t job = blockIdx.x; ok && job < P.jobs; job += nprog) {
-                const Job J = decode(P, job, CRTF);
+                const Job J = decode(P, cursor, job, CRTF);
                 const int64_t kb_total = J.I->kb_total, row_block = kb_total * kTileBytes;
                 const int nt = CRTF ? J.I->s : 1;
                 for (int tt = 0; ok && tt < nt; ++tt) {
@@ -196,8 +245,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_i8_modm_kernel(const __g
             uint32_t phase = 0;
             bool ok = !P.stall, issued = false;
             int local = 0;  // (job, chunk) pairs processed: selects the accumulator
+            ItemCursor cursor;
             for (int64_t job = blockIdx.x; ok && job < P.jobs; job += nprog) {
-                const Job J = decode(P, job, CRTF);
+                const Job J = decode(P, cursor, job, CRTF);
                 const int64_t kb_total = J.I->kb_total;
                 const int nt = CRTF ? J.I->s : 1;
                 for (int tt = 0; ok && tt < nt; ++tt)
@@ -254,17 +304,22 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_i8_modm_kernel(const __g
         constexpr int kChunks = BN / 32 / kEpiParts;  // 32-column chunks per warp
         int local = 0;
         bool ok = true;
+        ItemCursor cursor;
         for (int64_t job = blockIdx.x; ok && job < P.jobs; job += nprog) {
-            const Job J = decode(P, job, CRTF);
+            const Job J = decode(P, cursor, job, CRTF);
             const int nt = CRTF ? J.I->s : 1;
             for (int tt = 0; ok && tt < nt; ++tt) {
             const int t = CRTF ? tt : J.gt % J.I->s;
-            constexpr bool RES = KIND == kKindResidue || CRTF;
+            constexpr bool RES = KIND == kKindResidue || KIND == kKindShort || CRTF;
             const uint32_t m = RES ? J.I->mod_m[t] : 1u, mu = RES ? J.I->mod_mu[t] : 0u,
                            kbias = RES ? J.I->mod_kbias[t] : 0u;
             // at most kExactKB k-blocks (one chunk): |c| <= kExactSum, so u = c + kbias30 < 2^31 and
             // the multiply-high quotient is exact; otherwise Barrett with one correction step
+            // (item flag f32, at most 8 k-blocks: |c| <= 2^24 is exact in FP32, the quotient one FMA and the
+            // residue signed)
+            const bool f32 = KIND == kKindShort && J.I->f32;
             const bool exact = RES && J.I->kb_total <= kExactKB;
+            const float finv = __frcp_rn(static_cast<float>(m));
             const uint32_t kbias30 = RES ? J.I->mod_kbias30[t] : 0u, mx31 = RES ? J.I->mod_mx31[t] : 0u;
             const uint32_t mxs = RES ? J.I->mod_mxs[t] : 7u;
             const int64_t j = static_cast<int64_t>(J.tj) * kGemmJ + quarter * 32 + lane;
@@ -359,6 +414,23 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_i8_modm_kernel(const __g
                         dev::tmem_store_32x8(tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) +
                                                  static_cast<uint32_t>(2 * BN + 128 * half + 16 * tt + 8 * cc),
                                              w);
+                    } else if (KIND == kKindShort && f32) {
+                        if (j < nn && i0 < mm) {
+                            uint32_t w[8];
+                            if (m == 256u) {  // the residue is the low byte
+#pragma unroll
+                                for (int q = 0; q < 8; ++q)
+                                    w[q] = pack_low(cur[q], cur[q + 8], cur[q + 16], cur[q + 24]);
+                            } else {
+#pragma unroll
+                                for (int q = 0; q < 8; ++q)  // byte 4 q + b: row q + 8 b of the 32
+                                    w[q] = pack_low(residue_f32(cur[q], finv, 0u - m), residue_f32(cur[q + 8], finv, 0u - m),
+                                                    residue_f32(cur[q + 16], finv, 0u - m),
+                                                    residue_f32(cur[q + 24], finv, 0u - m));
+                            }
+                            *reinterpret_cast<uint4*>(blk) = make_uint4(w[0], w[1], w[2], w[3]);
+                            *reinterpret_cast<uint4*>(blk + 16) = make_uint4(w[4], w[5], w[6], w[7]);
+                        }
                     } else if (exact) {
                         if (j < nn && i0 < mm) {
                             uint32_t w[8];
@@ -490,11 +562,18 @@ void launch_bn(const GemmParams& P, int grid, cudaStream_t st) {
 
 }  // namespace
 
-cudaError_t prepare_gemm_kernels() {
+namespace {
+cudaError_t prepare_kernels() {
     cudaError_t e = cudaFuncSetAttribute(gemm_i8_modm_kernel<256, kKindResidue>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<256>::kSmemBytes);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(gemm_i8_modm_kernel<128, kKindResidue>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 Cfg<128>::kSmemBytes);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(gemm_i8_modm_kernel<256, kKindShort>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 Cfg<256>::kSmemBytes);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(gemm_i8_modm_kernel<128, kKindShort>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  Cfg<128>::kSmemBytes);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(gemm_i8_modm_kernel<256, kKindOz1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -507,6 +586,22 @@ cudaError_t prepare_gemm_kernels() {
                                  Cfg<128>::kSmemBytes);
     if (e == cudaSuccess) e = prepare_split_kernels();
     if (e == cudaSuccess) e = prepare_crt_kernels();
+    return e;
+}
+}  // namespace
+
+// The attributes last as long as the context: set once for each (a context's id is never used again),
+// which spares every later handle some forty driver calls.
+cudaError_t prepare_gemm_kernels() {
+    static std::mutex mutex;
+    static std::set<unsigned long long> done;  // a caller has made a runtime call: its context is current
+    CUcontext ctx = nullptr;
+    unsigned long long id = 0;
+    const bool known = cuCtxGetCurrent(&ctx) == CUDA_SUCCESS && ctx && cuCtxGetId(ctx, &id) == CUDA_SUCCESS;
+    std::lock_guard<std::mutex> lock(mutex);
+    if (known && done.count(id)) return cudaSuccess;
+    const cudaError_t e = prepare_kernels();
+    if (known && e == cudaSuccess) done.insert(id);
     return e;
 }
 
@@ -523,8 +618,14 @@ void launch_gemm(const GemmItem* d_items, int count, int64_t jobs, const GemmCon
     const GemmParams P = make_params(d_items, count, cfg.group_j > 0 ? cfg.group_j : 16, jobs, err);
     const int ctas = cfg.ctas > 0 ? std::min(cfg.ctas, num_sms) : num_sms;
     const int grid = static_cast<int>(std::min<int64_t>(ctas, jobs));
-    if (cfg.bn == 128) launch_bn<128>(P, grid, st);
-    else launch_bn<256>(P, grid, st);
+    if (cfg.has_short) {
+        if (cfg.bn == 128) launch_bn<128, kKindShort>(P, grid, st);
+        else launch_bn<256, kKindShort>(P, grid, st);
+    } else if (cfg.bn == 128) {
+        launch_bn<128>(P, grid, st);
+    } else {
+        launch_bn<256>(P, grid, st);
+    }
 }
 
 void launch_gemm_oz1(const GemmItem* d_items, int count, int64_t jobs, const GemmConfig& cfg, int num_sms, int* err,

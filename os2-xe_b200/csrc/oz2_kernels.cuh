@@ -101,6 +101,7 @@ struct GemmItem {
     int64_t pstride_i, pstride_j, rstride, ldr, m, n, kb_total;
     int64_t tiles, job0;
     int tiles_i, tiles_j, s, groups;
+    int f32;  // residues reduced in FP32 and signed (f32_residues)
     uint32_t mod_m[kMaxModuliExt], mod_mu[kMaxModuliExt], mod_kbias[kMaxModuliExt];
     uint32_t mod_kbias30[kMaxModuliExt], mod_mx31[kMaxModuliExt];  // exact quotient, kb_total <= kExactKB
     uint32_t mod_mxs[kMaxModuliExt];                                // its shift (oz2_plan.hpp)
@@ -139,6 +140,7 @@ struct CrtItem {
     double ar, ai, br, bi;
     double* C;
     int64_t block0, iblocks;  // blocks = ceil(ceil(n / cols) / jc) * iblocks, iblocks = ceil(m / 32)
+    int sgn;                  // the residues are signed (f32_residues)
     int cols, jc;             // a block: 32 rows x cols columns, jc times (crt_launch_shape)
 };
 
@@ -175,6 +177,7 @@ struct GemmConfig {
     int bn = 256;        // tile width along i (MMA N): 256 or 128
     int group_j = 16;    // raster: column tiles that share a row panel in flight
     int ctas = 0;        // persistent CTAs (0 = one per SM)
+    bool has_short = false;  // of a launch: some item's GemmItem::f32 is set
 };
 void launch_gemm(const GemmItem* d_items, int count, int64_t jobs, const GemmConfig& cfg, int num_sms, int* err,
                  cudaStream_t st);

@@ -216,6 +216,8 @@ extern "C" int oz2_dgemm_noalloc(void* stream, char ta, char tb, int64_t m, int6
     g.tiles = static_cast<int64_t>(g.tiles_i) * g.tiles_j;
     g.s = s;
     g.groups = 1;
+    g.f32 = f32_residues(p, kb_total) ? 1 : 0;
+    cfg.has_short = g.f32 != 0;
     g.job0 = 0;
     for (int t = 0; t < s; ++t) {
         g.mod_m[t] = mc[t].m;
@@ -236,6 +238,7 @@ extern "C" int oz2_dgemm_noalloc(void* stream, char ta, char tb, int64_t m, int6
     c.maxA = maxA;
     c.maxB = maxB;
     c.tk = p.tk;
+    c.sgn = g.f32;
     c.ar = alpha;
     c.br = beta;
     c.C = C;

@@ -197,6 +197,13 @@ int make_plan_ext(int s, int64_t k, Plan& p) {
     return 0;
 }
 
+bool f32_residues(const Plan& p, int64_t kb) {
+    if (kb > 8) return false;
+    for (int t = 0; t < p.s; ++t)
+        if (p.m[t] == 255 && kb > 4) return false;
+    return true;
+}
+
 int make_plan(int s, int64_t k, Plan& p) {
     if (s < 2 || s > kMaxModuli || k < 1) return 1;
     return make_plan_ext(s, k, p);

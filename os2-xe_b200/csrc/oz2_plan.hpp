@@ -100,6 +100,11 @@ struct Plan {
 // Returns 0, or 1 (invalid: s out of [2, 24], k < 1, s too small for k), or 5 (overflow).
 // ref src/ozaki2_gpu.hpp:159-200
 int make_plan(int s, int64_t k, Plan& p);
+// Whether the GEMM reduces this plan's sums over kb k-blocks in FP32, to signed residues (otherwise
+// in integers, to residues in [0, m)). |c| <= 128 * 128^2 kb must be exact in FP32: 8 k-blocks; m = 255, whose
+// signed residue must not reach +128, stays exact up to 4. B200, 4096^2, s = 16: the GEMM stage 196 ->
+// 159 us at k = 256, 163 -> 149 at 512, 224 -> 218 at 1024.
+bool f32_residues(const Plan& p, int64_t kb);
 // the same for s in [2, 32]: the reference's plans for s <= 24, the extended sets above
 int make_plan_ext(int s, int64_t k, Plan& p);
 // tk of make_plan_ext(s, k), or 0 where that plan is invalid (s too small for k)

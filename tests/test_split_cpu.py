@@ -1,4 +1,6 @@
-"""The split's two-instruction residue, exhaustively: for every modulus of every set and every byte
+"""The split's two-instruction residue and the GEMM epilogue's FP32 residue.
+
+The split's, exhaustively: for every modulus of every set and every byte
 dot product it can meet, the FP32 quotient leaves a byte congruent to the value in [-128, 127]."""
 import numpy as np
 import pytest
@@ -40,3 +42,23 @@ def test_symmetric_residue(m):
         assert r.min() >= -128 and r.max() <= 127
         assert np.array_equal(signed, r)
     assert np.all((signed - v) % m == 0)
+
+
+@pytest.mark.parametrize("m", moduli())
+def test_fp32_residue_of_gemm_sums(m):
+    """q = rint(fl(c fl(1/m))) in one rounding for every int32 sum of at most 1024 products (512 for m =
+    255), |c| <= 2^24 (2^23): c - q m is a byte in [-128, 127]. q does not decrease with c, so the sums on
+    both sides of every tie c = (j + 1/2) m and the ends of the range decide."""
+    top = 2 ** 23 if m == 255 else 2 ** 24
+    if m == 256:
+        return  # the residue is the low byte
+    j = np.arange(-top // m - 2, top // m + 2, dtype=np.int64)
+    c = np.concatenate([(2 * j + 1) * m // 2 + d for d in (-1, 0, 1, 2)] + [np.array([-top, -top + 1, 0, top - 1, top])])
+    c = c[np.abs(c) <= top]
+    num, e = int(np.float64(np.float32(1.0) / np.float32(m)) * 2.0 ** 32), 32
+    p = c * num
+    t = p >> e  # round to nearest even: the addend 1.5 2^23 is even, the sum's ulp 1
+    rest = p - (t << e)
+    t = t + ((rest > (1 << (e - 1))) | ((rest == (1 << (e - 1))) & (t % 2 == 1)))
+    r = c - t * m
+    assert r.min() >= -128 and r.max() <= 127
