@@ -590,18 +590,36 @@ cudaError_t prepare_kernels() {
 }
 }  // namespace
 
-// The attributes last as long as the context: set once for each (a context's id is never used again),
-// which spares every later handle some forty driver calls.
-cudaError_t prepare_gemm_kernels() {
-    static std::mutex mutex;
-    static std::set<unsigned long long> done;  // a caller has made a runtime call: its context is current
+// A number that no other context of the process ever has, or 0 when the driver does not say. The
+// driver's functions are looked up at run time: the library loads without a driver.
+static unsigned long long context_id() {
+    using GetCurrent = CUresult (*)(CUcontext*);
+    using GetId = CUresult (*)(CUcontext, unsigned long long*);
+    void *current = nullptr, *get_id = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPointByVersion("cuCtxGetCurrent", &current, 12000, cudaEnableDefault, &q) != cudaSuccess || !current ||
+        cudaGetDriverEntryPointByVersion("cuCtxGetId", &get_id, 12000, cudaEnableDefault, &q) != cudaSuccess || !get_id) {
+        cudaGetLastError();
+        return 0;
+    }
     CUcontext ctx = nullptr;
     unsigned long long id = 0;
-    const bool known = cuCtxGetCurrent(&ctx) == CUDA_SUCCESS && ctx && cuCtxGetId(ctx, &id) == CUDA_SUCCESS;
+    if (reinterpret_cast<GetCurrent>(current)(&ctx) != CUDA_SUCCESS || !ctx ||
+        reinterpret_cast<GetId>(get_id)(ctx, &id) != CUDA_SUCCESS)
+        return 0;
+    return id;
+}
+
+// The attributes last as long as the context: set once for each, which spares every later handle
+// some forty driver calls. Callers have made a runtime call, so their context is current.
+cudaError_t prepare_gemm_kernels() {
+    static std::mutex mutex;
+    static std::set<unsigned long long> done;
+    const unsigned long long id = context_id();
     std::lock_guard<std::mutex> lock(mutex);
-    if (known && done.count(id)) return cudaSuccess;
+    if (id && done.count(id)) return cudaSuccess;
     const cudaError_t e = prepare_kernels();
-    if (known && e == cudaSuccess) done.insert(id);
+    if (id && e == cudaSuccess) done.insert(id);
     return e;
 }
 
