@@ -684,14 +684,21 @@ void issue(oz2_context* h, const Program& prog, const unsigned char* dev) {
 }
 
 // ---------------------------------------------------------------- GEMM configuration
-GemmConfig heuristic_config(const std::vector<const Prob*>& probs) {
+GemmConfig heuristic_config(const std::vector<const Prob*>& probs, int num_sms) {
     GemmConfig c;
-    // narrow problems waste less padding with 128-row tiles along i
-    std::vector<int64_t> ms;
-    for (auto* p : probs) ms.push_back(p->m);
-    std::sort(ms.begin(), ms.end());
-    const int64_t med = ms.empty() ? 0 : ms[ms.size() / 2];
-    c.bn = med > 0 && med <= 384 ? 128 : 256;
+    // The tile's width along i by the work of the padded tiles: a 128-row tile costs about 0.8 of a 256-row
+    // one (it reads twice the shared-memory bytes per multiply-add; B200, 4096 x 300 x 700, 6000^2 x 384,
+    // 2048^3: 0.64 to 0.83), so 128 only pays where most of the work lies in problems of at most 128 rows.
+    // 512 grouped problems: GEMM stage 1594 us with 256, 2040 with 128; 300 x 4000 x 700: 32 and 40.
+    // Or where all its tiles run at once (256^3, s = 16: 9 and 10 us).
+    double w128 = 0.0, w256 = 0.0, jobs = 0.0;
+    for (auto* p : probs) {
+        jobs += static_cast<double>(p->G) * p->plan->s * gemm_tiles_i(p->m, 128) * ceil_div(p->n, kGemmJ);
+        const double w = static_cast<double>(p->G) * p->plan->s * ceil_div(p->n, kGemmJ) * ceil_div(p->k, kTileK);
+        w128 += 0.8 * w * gemm_tiles_i(p->m, 128);
+        w256 += w * gemm_tiles_i(p->m, 256);
+    }
+    c.bn = w128 < w256 || jobs <= num_sms ? 128 : 256;
     c.group_j = 16;
     return c;
 }
@@ -711,7 +718,7 @@ GemmConfig config_for(oz2_context* h, const std::vector<const Prob*>& probs) {
     if (h->has_forced) return h->forced;
     auto it = h->tuned.find(shape_signature(probs));
     if (it != h->tuned.end()) return it->second;
-    return heuristic_config(probs);
+    return heuristic_config(probs, h->num_sms);
 }
 
 // ---------------------------------------------------------------- one emulated GEMM (tiled)
@@ -2437,7 +2444,7 @@ int oz2_autotune_grouped(oz2_handle h, int count, const oz2_dgemm_problem* probl
     std::vector<GemmConfig> cands;
     for (int bn : {256, 128})
         for (int gj : {4, 8, 16, 32}) cands.push_back(GemmConfig{bn, gj, 0});
-    GemmConfig best = heuristic_config(bp);
+    GemmConfig best = heuristic_config(bp, h->num_sms);
     double best_ms = std::numeric_limits<double>::infinity();
     h->forced = best;
     h->has_forced = true;

@@ -43,7 +43,20 @@ namespace {
 constexpr uint32_t kBarBytes = 256;
 constexpr int kEpiWarps = 8;                       // two per TMEM lane quarter (four measured slower)
 constexpr int kEpiParts = kEpiWarps / 4;           // column ranges of the accumulator
-constexpr int kGemmThreads = 64 + 32 * kEpiWarps;  // producer, MMA issuer, epilogue
+constexpr int kJobBatch = 32;                      // jobs the scheduler decodes at a time
+
+struct Job {
+    const GemmItem* I;  // null past the CTA's last job
+    const int8_t *srcJ, *srcI;  // the job's first plane tiles (kKindCrt: of modulus 0)
+    uint8_t* out;               // residues of its first 32 rows and first column
+    int64_t out_step;           // from one 32-row block to the next
+    int gt, t;                  // group * s + modulus; modulus
+    int ti, tj, kb, nch;        // tile; k blocks; k chunks
+    int ileft, jleft;           // rows and columns from the tile's first on
+    uint32_t m, mu, kbias, kbias30, mx31, mxs;  // the modulus's constants
+    int f32;
+};
+constexpr uint32_t kJobBytes = 2 * kJobBatch * sizeof(Job);
 
 template <int BN>
 struct Cfg {
@@ -68,59 +81,6 @@ struct GemmParams {
     int crt_shift;     // limbs moved up by this many bits to end at the fourth
 };
 
-struct Job {
-    const GemmItem* I;
-    int gt;  // group * s + modulus
-    int ti, tj;
-    int64_t nch;  // k chunks
-};
-// The items of a role's increasing job numbers: one search for the first, then a step forward now
-// and then; the next item's first job is kept, so a job of the same item reads nothing.
-struct ItemCursor {
-    int item = 0;
-    int64_t next = -1;  // first job of item + 1 (-1: not searched yet)
-    __device__ __forceinline__ void find(const GemmItem* items, int count, int64_t job) {
-        if (next < 0) {
-            int hi = count - 1;
-            while (item < hi) {
-                const int mid = (item + hi + 1) >> 1;
-                if (items[mid].job0 <= job) item = mid;
-                else hi = mid - 1;
-            }
-        } else {
-            if (job < next) return;
-            ++item;
-            while (item + 1 < count && items[item + 1].job0 <= job) ++item;
-        }
-        next = item + 1 < count ? items[item + 1].job0 : INT64_MAX;
-    }
-};
-// per_tile: the job is a tile and runs every modulus (kKindCrt); otherwise (group, modulus, tile)
-__device__ __forceinline__ Job decode(const GemmParams& P, ItemCursor& cur, int64_t job, bool per_tile = false) {
-    cur.find(P.items, P.count, job);
-    Job J;
-    J.I = P.items + cur.item;
-    // 32-bit arithmetic: an item's jobs (groups * s * tiles) are bounded by its residue planes,
-    // s m n bytes of device memory, so they stay far below 2^32 (one 64-bit division costs
-    // several times a 32-bit one, and every warp decodes every job)
-    const uint32_t local = static_cast<uint32_t>(job - J.I->job0);
-    const uint32_t tiles = static_cast<uint32_t>(J.I->tiles);
-    const uint32_t gt = per_tile ? 0u : local / tiles;
-    J.gt = static_cast<int>(gt);
-    const uint32_t tile = local - gt * tiles;
-    const uint32_t tiles_i = static_cast<uint32_t>(J.I->tiles_i), tiles_j = static_cast<uint32_t>(J.I->tiles_j);
-    const uint32_t group_j = static_cast<uint32_t>(P.group_j);
-    const uint32_t per_grp = group_j * tiles_i;
-    const uint32_t grp = tile / per_grp, rem = tile - grp * per_grp;
-    const uint32_t first_j = grp * group_j;
-    const uint32_t gj = min(group_j, tiles_j - first_j);
-    const uint32_t qj = rem / gj;
-    J.tj = static_cast<int>(first_j + (rem - qj * gj));
-    J.ti = static_cast<int>(qj);
-    J.nch = (J.I->kb_total + kChunkKB - 1) / kChunkKB;
-    return J;
-}
-
 // KIND: kKindResidue the Ozaki-II GEMM (int8 planes, residues mod m); kKindOz1 the Ozaki Scheme I
 // baseline (job t = digit pair, int64 atomic sums per anti-diagonal instead of residues);
 // kKindCert the certificate (bf16 planes of scaled magnitudes, kind::f16 MMAs, the largest
@@ -131,7 +91,17 @@ __device__ __forceinline__ Job decode(const GemmParams& P, ItemCursor& cur, int6
 // its 64 entries per lane and writes C)
 // kKindShort as kKindResidue for launches with items of few k-blocks (GemmItem::f32), beside which others may
 // run; launches without them take the kernel without that code, which measured 0.5 % faster at long k
-constexpr int kKindResidue = 0, kKindOz1 = 1, kKindCert = 2, kKindCrt = 3, kKindShort = 4;
+// kKindQueue kKindShort with a scheduler warp that decodes 32 jobs at a time for the other roles: at few
+// k-blocks a job is shorter than the chain of item-table loads and divisions that finds it. B200, 4096^2 x
+// 256, s = 16: 161 -> 132 us; 512 grouped problems 2039 -> 1827. For launches of at least kQueueRounds jobs
+// per CTA: below, its first batch only adds latency (512^3 12.4 -> 14.5 us). At long k every role decodes
+// its own jobs (the extra warp measured 1.3 % slower there, 4096^2 x 2048 376 -> 382 us).
+constexpr int kKindResidue = 0, kKindOz1 = 1, kKindCert = 2, kKindCrt = 3, kKindShort = 4, kKindQueue = 5;
+constexpr int kQueueRounds = 8;
+template <int KIND>
+__host__ __device__ constexpr int gemm_threads() { return 64 + 32 * kEpiWarps + (KIND == kKindQueue ? 32 : 0); }
+template <int BN, int KIND>
+constexpr int gemm_smem() { return Cfg<BN>::kSmemBytes + (KIND == kKindQueue ? static_cast<int>(kJobBytes) : 0); }
 
 // low bytes of a, b, c, d as one little-endian word
 __device__ __forceinline__ uint32_t pack_low(uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
@@ -154,8 +124,55 @@ __device__ __forceinline__ uint32_t residue_f32(uint32_t c, float finv, uint32_t
     return r;
 }
 
+// Job number -> item, modulus and tile (kKindCrt: a job is a tile and runs every modulus)
 template <int BN, int KIND>
-__global__ void __launch_bounds__(kGemmThreads, 1) gemm_i8_modm_kernel(const __grid_constant__ GemmParams P) {
+__device__ __forceinline__ void decode(const GemmParams& P, int64_t job, Job& J) {
+    constexpr bool OZ1 = KIND == kKindOz1, CERT = KIND == kKindCert, CRTF = KIND == kKindCrt;
+    int lo = 0, hi = P.count - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (P.items[mid].job0 <= job) lo = mid;
+        else hi = mid - 1;
+    }
+    const GemmItem* __restrict__ I = P.items + lo;
+    // 32-bit arithmetic: an item's jobs (groups * s * tiles) are bounded by its residue planes,
+    // s m n bytes of device memory, so they stay far below 2^32
+    const uint32_t local = static_cast<uint32_t>(job - I->job0), tiles = static_cast<uint32_t>(I->tiles);
+    const uint32_t gt = CRTF ? 0u : local / tiles, tile = local - gt * tiles;
+    const uint32_t tiles_i = static_cast<uint32_t>(I->tiles_i), tiles_j = static_cast<uint32_t>(I->tiles_j);
+    const uint32_t group_j = static_cast<uint32_t>(P.group_j), per_grp = group_j * tiles_i;
+    const uint32_t grp = tile / per_grp, rem = tile - grp * per_grp;
+    const uint32_t first_j = grp * group_j, gj = min(group_j, tiles_j - first_j), qj = rem / gj;
+    const int tj = static_cast<int>(first_j + (rem - qj * gj)), ti = static_cast<int>(qj);
+    const int64_t kb_total = I->kb_total, row_block = kb_total * kTileBytes;
+    const int pj = OZ1 ? I->pair_b[gt] : gt, pi = OZ1 ? I->pair_a[gt] : gt;
+    J.srcJ = I->planes_j + pj * I->pstride_j + tj * row_block;
+    J.srcI = I->planes_i + pi * I->pstride_i + (static_cast<int64_t>(ti) * (BN / 128)) * row_block;
+    J.gt = static_cast<int>(gt);
+    J.t = static_cast<int>(gt) % I->s;
+    J.ti = ti;
+    J.tj = tj;
+    J.kb = static_cast<int>(kb_total);
+    J.nch = static_cast<int>((kb_total + kChunkKB - 1) / kChunkKB);
+    const int64_t ileft = I->m - static_cast<int64_t>(ti) * BN, jleft = I->n - static_cast<int64_t>(tj) * kGemmJ;
+    J.ileft = static_cast<int>(min(ileft, int64_t{BN}));
+    J.jleft = static_cast<int>(min(jleft, int64_t{kGemmJ}));
+    if constexpr (!OZ1 && !CERT && !CRTF) {
+        J.out_step = 32 * I->n;
+        J.out = I->resid + J.gt * I->rstride + static_cast<int64_t>(tj) * (32 * kGemmJ) + ti * (BN / 32) * J.out_step;
+        J.m = I->mod_m[J.t];
+        J.mu = I->mod_mu[J.t];
+        J.kbias = I->mod_kbias[J.t];
+        J.kbias30 = I->mod_kbias30[J.t];
+        J.mx31 = I->mod_mx31[J.t];
+        J.mxs = I->mod_mxs[J.t];
+        J.f32 = I->f32;
+    }
+    J.I = I;
+}
+
+template <int BN, int KIND>
+__global__ void __launch_bounds__(gemm_threads<KIND>(), 1) gemm_i8_modm_kernel(const __grid_constant__ GemmParams P) {
     constexpr bool OZ1 = KIND == kKindOz1, CERT = KIND == kKindCert, CRTF = KIND == kKindCrt;
     static_assert(!CRTF || BN == 128, "the fused CRT keeps its residues beside two 128-column accumulators");
     using C = Cfg<BN>;
@@ -163,14 +180,17 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_i8_modm_kernel(const __g
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t{1023});
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::kStages * C::kStageBytes);
-    // barriers: full[kStages] empty[kStages] acc_full[2] acc_empty[2] drain
+    // barriers: full[kStages] empty[kStages] acc_full[2] acc_empty[2] drain jobs_full[2] jobs_empty[2]
     const uint32_t bar0 = dev::smem_addr(bars);
     auto full = [&](int i) { return bar0 + 8u * i; };
     auto empty = [&](int i) { return bar0 + 8u * (C::kStages + i); };
     auto acc_full = [&](int a) { return bar0 + 8u * (2 * C::kStages + a); };
     auto acc_empty = [&](int a) { return bar0 + 8u * (2 * C::kStages + 2 + a); };
     const uint32_t drain = bar0 + 8u * (2 * C::kStages + 4);
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * C::kStages + 5);
+    auto jobs_full = [&](int b) { return bar0 + 8u * (2 * C::kStages + 5 + b); };
+    auto jobs_empty = [&](int b) { return bar0 + 8u * (2 * C::kStages + 7 + b); };
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * C::kStages + 9);
+    Job* job_ring = reinterpret_cast<Job*>(smem + C::kStages * C::kStageBytes + kBarBytes);  // two batches
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -182,6 +202,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_i8_modm_kernel(const __g
         for (int a = 0; a < 2; ++a) {
             dev::mbar_init(acc_full(a), 1);
             dev::mbar_init(acc_empty(a), kEpiWarps);
+            dev::mbar_init(jobs_full(a), 1);
+            dev::mbar_init(jobs_empty(a), 2 + kEpiWarps);  // producer, MMA issuer, epilogue warps
         }
         dev::mbar_init(drain, 1);
         *abort_flag = 0;
@@ -195,24 +217,70 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_i8_modm_kernel(const __g
     __syncthreads();
     dev::tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    // The CTA's n-th job for one role: false past the last job, or (ok false) when the wait for its batch ran
+    // out; one lane waits (`whole` roles are a warp). job_done(n) releases the batch after its last job.
+    constexpr bool SCHED = KIND == kKindQueue;
     const int64_t nprog = gridDim.x;
+    auto job_at = [&](int n, bool whole, Job& J, bool& ok) -> bool {
+        if constexpr (SCHED) {
+            if ((n & (kJobBatch - 1)) == 0) {
+                const int b = (n / kJobBatch) & 1;
+                int w = 1;
+                if (!whole || lane == 0)
+                    w = dev::mbar_wait(jobs_full(b), (n / (2 * kJobBatch)) & 1u, abort_flag, P.err, dev::kErrTimeoutJobs, P.wait_ns);
+                if (whole) w = __shfl_sync(0xFFFFFFFFu, w, 0);
+                if (!w) {
+                    ok = false;
+                    return false;
+                }
+            }
+            J = job_ring[n & (2 * kJobBatch - 1)];
+            return J.I != nullptr;
+        } else {
+            const int64_t job = blockIdx.x + n * nprog;
+            if (job >= P.jobs) return false;
+            decode<BN, KIND>(P, job, J);
+            return true;
+        }
+    };
+    auto job_done = [&](int n, bool whole) {
+        if (!SCHED || (n & (kJobBatch - 1)) != kJobBatch - 1) return;
+        if (whole) __syncwarp();
+        if (!whole || lane == 0) dev::mbar_arrive(jobs_empty((n / kJobBatch) & 1));
+    };
 
-    if (warp == 0) {
+    if (SCHED && warp == 2 + kEpiWarps) {
+        // scheduler: a batch of jobs at a time, one per lane, two batches ahead at most
+        for (int b = 0;; ++b) {
+            int w = 1;
+            if (lane == 0)
+                w = dev::mbar_wait(jobs_empty(b & 1), ((b >> 1) & 1u) ^ 1u, abort_flag, P.err, dev::kErrTimeoutJobs, P.wait_ns);
+            if (!__shfl_sync(0xFFFFFFFFu, w, 0)) break;
+            const int64_t job = blockIdx.x + (static_cast<int64_t>(b) * kJobBatch + lane) * nprog;
+            Job& J = job_ring[(b & 1) * kJobBatch + lane];
+            if (job < P.jobs) decode<BN, KIND>(P, job, J);
+            else J.I = nullptr;
+            __syncwarp();
+            if (lane == 0) dev::mbar_arrive(jobs_full(b & 1));
+            if (__any_sync(0xFFFFFFFFu, job >= P.jobs)) break;  // the batch ends the CTA's jobs
+        }
+    } else if (warp == 0) {
         if (lane == 0) {
             int stage = 0;
             uint32_t phase = 0;
             uint32_t issued_mask = 0, issued_phase = 0;
             bool ok = true;
-            ItemCursor cursor;
-            for (int64_t job = blockIdx.x; ok && job < P.jobs; job += nprog) {
-                const Job J = decode(P, cursor, job, CRTF);
-                const int64_t kb_total = J.I->kb_total, row_block = kb_total * kTileBytes;
+            for (int n = 0;; ++n) {
+                Job J;
+                if (!job_at(n, false, J, ok)) break;
+                const int64_t kb_total = J.kb, row_block = kb_total * kTileBytes;
+                const int8_t *srcJ = J.srcJ, *srcI = J.srcI;
                 const int nt = CRTF ? J.I->s : 1;
                 for (int tt = 0; ok && tt < nt; ++tt) {
-                const int gt = CRTF ? tt : J.gt;
-                const int pj = OZ1 ? J.I->pair_b[gt] : gt, pi = OZ1 ? J.I->pair_a[gt] : gt;
-                const int8_t* srcJ = J.I->planes_j + pj * J.I->pstride_j + J.tj * row_block;
-                const int8_t* srcI = J.I->planes_i + pi * J.I->pstride_i + (static_cast<int64_t>(J.ti) * (BN / 128)) * row_block;
+                if (CRTF && tt) {
+                    srcJ += J.I->pstride_j;
+                    srcI += J.I->pstride_i;
+                }
                 for (int64_t kb = 0; ok && kb < kb_total; ++kb) {
                     if (!dev::mbar_wait(empty(stage), phase ^ 1u, abort_flag, P.err, dev::kErrTimeoutEmpty,
                                          P.wait_ns)) {
@@ -233,6 +301,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_i8_modm_kernel(const __g
                     }
                 }
                 }
+                if (!ok) break;
+                job_done(n, false);
             }
             if (!ok) {  // let every copy that was issued land before the CTA exits
                 for (int i = 0; i < C::kStages; ++i)
@@ -245,13 +315,13 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_i8_modm_kernel(const __g
             uint32_t phase = 0;
             bool ok = !P.stall, issued = false;
             int local = 0;  // (job, chunk) pairs processed: selects the accumulator
-            ItemCursor cursor;
-            for (int64_t job = blockIdx.x; ok && job < P.jobs; job += nprog) {
-                const Job J = decode(P, cursor, job, CRTF);
-                const int64_t kb_total = J.I->kb_total;
-                const int nt = CRTF ? J.I->s : 1;
+            for (int n = 0; ok; ++n) {
+                Job J;
+                if (!job_at(n, false, J, ok)) break;
+                const int64_t kb_total = J.kb;
+                const int nch = J.nch, nt = CRTF ? J.I->s : 1;
                 for (int tt = 0; ok && tt < nt; ++tt)
-                for (int64_t c = 0; ok && c < J.nch; ++c, ++local) {
+                for (int64_t c = 0; ok && c < nch; ++c, ++local) {
                     const int acc = local & 1;
                     const uint32_t use = static_cast<uint32_t>(local >> 1);
                     if (!dev::mbar_wait(acc_empty(acc), (use & 1u) ^ 1u, abort_flag, P.err, dev::kErrTimeoutAccEmpty,
@@ -292,6 +362,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_i8_modm_kernel(const __g
                     if (!ok) break;
                     dev::tc_commit(acc_full(acc));
                 }
+                if (ok) job_done(n, false);
             }
             if (!ok && issued) {  // wait until every MMA issued so far has completed
                 dev::tc_commit(drain);
@@ -304,31 +375,32 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_i8_modm_kernel(const __g
         constexpr int kChunks = BN / 32 / kEpiParts;  // 32-column chunks per warp
         int local = 0;
         bool ok = true;
-        ItemCursor cursor;
-        for (int64_t job = blockIdx.x; ok && job < P.jobs; job += nprog) {
-            const Job J = decode(P, cursor, job, CRTF);
+        for (int n = 0; ok; ++n) {
+            Job J;
+            if (!job_at(n, true, J, ok)) break;
             const int nt = CRTF ? J.I->s : 1;
             for (int tt = 0; ok && tt < nt; ++tt) {
-            const int t = CRTF ? tt : J.gt % J.I->s;
-            constexpr bool RES = KIND == kKindResidue || KIND == kKindShort || CRTF;
-            const uint32_t m = RES ? J.I->mod_m[t] : 1u, mu = RES ? J.I->mod_mu[t] : 0u,
-                           kbias = RES ? J.I->mod_kbias[t] : 0u;
+            const int t = CRTF ? tt : J.t;
+            constexpr bool SHORT = KIND == kKindShort || KIND == kKindQueue;
+            constexpr bool RES = KIND == kKindResidue || SHORT || CRTF;
+            const uint32_t m = CRTF ? J.I->mod_m[t] : (RES ? J.m : 1u), mu = J.mu, kbias = J.kbias;
             // at most kExactKB k-blocks (one chunk): |c| <= kExactSum, so u = c + kbias30 < 2^31 and
             // the multiply-high quotient is exact; otherwise Barrett with one correction step
             // (item flag f32, at most 8 k-blocks: |c| <= 2^24 is exact in FP32, the quotient one FMA and the
             // residue signed)
-            const bool f32 = KIND == kKindShort && J.I->f32;
-            const bool exact = RES && J.I->kb_total <= kExactKB;
+            const bool f32 = SHORT && J.f32;
+            const bool exact = RES && J.kb <= kExactKB;
             const float finv = __frcp_rn(static_cast<float>(m));
-            const uint32_t kbias30 = RES ? J.I->mod_kbias30[t] : 0u, mx31 = RES ? J.I->mod_mx31[t] : 0u;
-            const uint32_t mxs = RES ? J.I->mod_mxs[t] : 7u;
+            const uint32_t kbias30 = CRTF ? J.I->mod_kbias30[t] : J.kbias30, mx31 = CRTF ? J.I->mod_mx31[t] : J.mx31;
+            const uint32_t mxs = CRTF ? J.I->mod_mxs[t] : J.mxs;
             const int64_t j = static_cast<int64_t>(J.tj) * kGemmJ + quarter * 32 + lane;
-            const int64_t mm = J.I->m, nn = J.I->n;
-            uint8_t* rowj = RES && !CRTF ? J.I->resid + J.gt * J.I->rstride + j * 32 : nullptr;  // + (i / 32) * 32 n
+            const bool jin = quarter * 32 + lane < J.jleft;
+            const int64_t mm = CERT || OZ1 ? J.I->m : 0, nn = CERT || OZ1 ? J.I->n : 0;
+            uint8_t* rowj = J.out + (quarter * 32 + lane) * 32;  // + 32-row block * out_step
             // certificate: this lane's column sum (zero for a padding column or an all-zero column,
             // whose entries are skipped)
             const float sj = CERT && j < nn ? static_cast<float>(J.I->cert_sb[j]) : 0.0f;
-            for (int64_t c = 0; c < J.nch; ++c, ++local) {
+            for (int c = 0; c < J.nch; ++c, ++local) {
                 const int acc = local & 1;
                 const uint32_t use = static_cast<uint32_t>(local >> 1);
                 int w_ok = 1;
@@ -352,7 +424,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_i8_modm_kernel(const __g
                     // the next chunk's load is in flight during this chunk's arithmetic
                     if (cc + 1 < kChunks) dev::tmem_load_32x32(taddr + (cc + 1) * 32, v[(cc + 1) & 1]);
                     const int64_t i0 = static_cast<int64_t>(J.ti) * BN + (half * kChunks + cc) * 32;
-                    uint8_t* blk = rowj + (i0 >> 5) * (32 * nn);  // this chunk's 32 bytes of row j
+                    uint8_t* blk = rowj + (half * kChunks + cc) * J.out_step;  // this chunk's 32 bytes of row j
+                    const bool rin = jin && (half * kChunks + cc) * 32 < J.ileft;
                     if constexpr (CERT) {
                         // the warp's 32 lanes are 32 consecutive j of one adaptive tile column
                         // (cert_tile is a multiple of 128), its 32 columns i0.. one tile row
@@ -414,8 +487,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_i8_modm_kernel(const __g
                         dev::tmem_store_32x8(tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) +
                                                  static_cast<uint32_t>(2 * BN + 128 * half + 16 * tt + 8 * cc),
                                              w);
-                    } else if (KIND == kKindShort && f32) {
-                        if (j < nn && i0 < mm) {
+                    } else if (SHORT && f32) {
+                        if (rin) {
                             uint32_t w[8];
                             if (m == 256u) {  // the residue is the low byte
 #pragma unroll
@@ -432,7 +505,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_i8_modm_kernel(const __g
                             *reinterpret_cast<uint4*>(blk + 16) = make_uint4(w[4], w[5], w[6], w[7]);
                         }
                     } else if (exact) {
-                        if (j < nn && i0 < mm) {
+                        if (rin) {
                             uint32_t w[8];
 #pragma unroll
                             for (int q = 0; q < 8; ++q) {
@@ -448,7 +521,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_i8_modm_kernel(const __g
                             *reinterpret_cast<uint4*>(blk) = make_uint4(w[0], w[1], w[2], w[3]);
                             *reinterpret_cast<uint4*>(blk + 16) = make_uint4(w[4], w[5], w[6], w[7]);
                         }
-                    } else if (j < nn && i0 < mm) {
+                    } else if (rin) {
                         uint32_t ow[8] = {0, 0, 0, 0, 0, 0, 0, 0};
                         if (accumulate) {
                             const uint4 o0 = *reinterpret_cast<const uint4*>(blk);
@@ -535,6 +608,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_i8_modm_kernel(const __g
                     dev::tc_fence_before();
                 }
             }
+            if (ok) job_done(n, true);
         }
         if constexpr (CRTF) dev::tmem_store_wait();  // no residue store in flight when TMEM is freed
     }
@@ -557,33 +631,27 @@ GemmParams make_params(const GemmItem* d_items, int count, int group_j, int64_t 
 
 template <int BN, int KIND = kKindResidue>
 void launch_bn(const GemmParams& P, int grid, cudaStream_t st) {
-    gemm_i8_modm_kernel<BN, KIND><<<grid, kGemmThreads, Cfg<BN>::kSmemBytes, st>>>(P);
+    gemm_i8_modm_kernel<BN, KIND><<<grid, gemm_threads<KIND>(), gemm_smem<BN, KIND>(), st>>>(P);
 }
 
 }  // namespace
 
 namespace {
+template <int BN, int KIND>
+cudaError_t prepare_kernel() {
+    return cudaFuncSetAttribute(gemm_i8_modm_kernel<BN, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, gemm_smem<BN, KIND>());
+}
+
 cudaError_t prepare_kernels() {
-    cudaError_t e = cudaFuncSetAttribute(gemm_i8_modm_kernel<256, kKindResidue>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<256>::kSmemBytes);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(gemm_i8_modm_kernel<128, kKindResidue>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 Cfg<128>::kSmemBytes);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(gemm_i8_modm_kernel<256, kKindShort>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 Cfg<256>::kSmemBytes);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(gemm_i8_modm_kernel<128, kKindShort>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 Cfg<128>::kSmemBytes);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(gemm_i8_modm_kernel<256, kKindOz1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 Cfg<256>::kSmemBytes);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(gemm_i8_modm_kernel<256, kKindCert>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 Cfg<256>::kSmemBytes);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(gemm_i8_modm_kernel<128, kKindCrt>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 Cfg<128>::kSmemBytes);
+    cudaError_t e = prepare_kernel<256, kKindResidue>();
+    if (e == cudaSuccess) e = prepare_kernel<128, kKindResidue>();
+    if (e == cudaSuccess) e = prepare_kernel<256, kKindShort>();
+    if (e == cudaSuccess) e = prepare_kernel<128, kKindShort>();
+    if (e == cudaSuccess) e = prepare_kernel<256, kKindQueue>();
+    if (e == cudaSuccess) e = prepare_kernel<128, kKindQueue>();
+    if (e == cudaSuccess) e = prepare_kernel<256, kKindOz1>();
+    if (e == cudaSuccess) e = prepare_kernel<256, kKindCert>();
+    if (e == cudaSuccess) e = prepare_kernel<128, kKindCrt>();
     if (e == cudaSuccess) e = prepare_split_kernels();
     if (e == cudaSuccess) e = prepare_crt_kernels();
     return e;
@@ -636,7 +704,10 @@ void launch_gemm(const GemmItem* d_items, int count, int64_t jobs, const GemmCon
     const GemmParams P = make_params(d_items, count, cfg.group_j > 0 ? cfg.group_j : 16, jobs, err);
     const int ctas = cfg.ctas > 0 ? std::min(cfg.ctas, num_sms) : num_sms;
     const int grid = static_cast<int>(std::min<int64_t>(ctas, jobs));
-    if (cfg.has_short) {
+    if (cfg.has_short && jobs >= static_cast<int64_t>(kQueueRounds) * grid) {
+        if (cfg.bn == 128) launch_bn<128, kKindQueue>(P, grid, st);
+        else launch_bn<256, kKindQueue>(P, grid, st);
+    } else if (cfg.has_short) {
         if (cfg.bn == 128) launch_bn<128, kKindShort>(P, grid, st);
         else launch_bn<256, kKindShort>(P, grid, st);
     } else if (cfg.bn == 128) {

@@ -199,7 +199,8 @@ extern "C" int oz2_dgemm_noalloc(void* stream, char ta, char tb, int64_t m, int6
         split_geometry(sp, 0);
     }
     GemmConfig cfg;
-    cfg.bn = m <= 384 ? 128 : 256;
+    // as oz2_dgemm's choice for one problem
+    cfg.bn = m <= 128 || s * gemm_tiles_i(m, 128) * ceil_div(n, kGemmJ) <= num_sms ? 128 : 256;
     GemmItem& g = T.g;
     g.planes_i = planesA;
     g.planes_j = planesB;

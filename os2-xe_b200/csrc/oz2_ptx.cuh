@@ -10,7 +10,7 @@ namespace dev {
 
 // Device-side error codes written to the handle's error word (host maps them to OZ2_ETIMEOUT).
 enum : int { kErrNone = 0, kErrTimeoutFull = 1, kErrTimeoutEmpty = 2, kErrTimeoutAccFull = 3,
-             kErrTimeoutAccEmpty = 4, kErrTimeoutDrain = 5 };
+             kErrTimeoutAccEmpty = 4, kErrTimeoutDrain = 5, kErrTimeoutJobs = 6 };
 
 // A wait on an mbarrier phase that is still pending after this long is treated as a fault.
 // Healthy waits last microseconds. The GEMM takes its limit as a kernel parameter (this value
