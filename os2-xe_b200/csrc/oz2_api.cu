@@ -375,20 +375,25 @@ int64_t crt_geom(CrtItem& it, int64_t b0) { return crt_item_blocks(it, b0); }
 
 // Appends split, GEMM and CRT operations for a list of tasks (launches grouped by kernel variant)
 void plan_tasks(Program& prog, const std::vector<Task>& tasks, const GemmConfig& cfg) {
-    // split: group by (row_contig, complex / fused scale, limb path: narrow, wide, widest)
+    // split: group by (complex / fused scale, limb path: narrow, wide, widest), and by layout where the kernel
+    // is one layout's (the fused and the tensor-core split); 128^3: one launch 6 us, one per layout 11 us
     std::map<std::tuple<int, int, int>, std::vector<SplitItem>> split_groups;
+    auto add_split = [&](const SplitItem& it, int wide) {
+        const int layout = it.fuse || (!it.cplx && split_path()) ? it.row_contig : 0;
+        split_groups[{layout, it.cplx + 2 * it.fuse, wide}].push_back(it);
+    };
     for (const Task& t : tasks) {
         const Prob& p = *t.p;
         const int wide = p.plan->tk > kWideScaleBits ? 2 : (p.plan->tk > kNarrowScaleBits ? 1 : 0);
         if (t.split_b) {
             SplitItem it = side_item(p, false, t.j0, t.nb, t.maxB, t.planesB);
             it.fuse = t.fuse_b;
-            split_groups[{it.row_contig, it.cplx + 2 * it.fuse, wide}].push_back(it);
+            add_split(it, wide);
         }
         if (t.split_a) {
             SplitItem it = side_item(p, true, t.i0, t.mb, t.maxA, t.planesA);
             it.fuse = t.fuse_a;
-            split_groups[{it.row_contig, it.cplx + 2 * it.fuse, wide}].push_back(it);
+            add_split(it, wide);
         }
     }
     for (auto& kv : split_groups) split_launch_shape(kv.second.data(), static_cast<int>(kv.second.size()));
@@ -525,9 +530,8 @@ void plan_tasks(Program& prog, const std::vector<Task>& tasks, const GemmConfig&
 }
 
 void plan_scale(oz2_context* h, Program& prog, std::vector<ScaleItem>& items) {
-    // group by (row_contig, complex)
-    std::map<std::pair<int, int>, std::vector<ScaleItem>> groups;
-    for (auto& it : items) groups[{it.row_contig, it.cplx}].push_back(it);
+    std::map<int, std::vector<ScaleItem>> groups;  // real, complex
+    for (auto& it : items) groups[it.cplx].push_back(it);
     for (auto& kv : groups) {
         int64_t blocks = 0;
         for (auto& it : kv.second) blocks += scale_item_blocks(it, h->num_sms, blocks);
@@ -640,13 +644,11 @@ int read_back(oz2_context* h, std::initializer_list<HostRead> reads) {
     return OZ2_OK;
 }
 
-int upload(oz2_context* h, const Program& prog, unsigned char* dev) {
-    return put_blob(h, prog.blob.data(), prog.blob.size(), dev);
-}
-
-void issue(oz2_context* h, const Program& prog, const unsigned char* dev) {
+// `filled`: a Memset that the launch before this one made
+void issue(oz2_context* h, const Program& prog, const unsigned char* dev, const Op* filled = nullptr) {
     const unsigned char* hb = prog.blob.data();
     for (const Op& op : prog.ops) {
+        if (&op == filled) continue;
         if (op.kind != Op::Mark) ++h->launches;
         switch (op.kind) {
             case Op::Memset: launch_fill(op.ptr, 0, op.bytes, h->stream); break;
@@ -681,6 +683,23 @@ void issue(oz2_context* h, const Program& prog, const unsigned char* dev) {
             case Op::Mark: mark(h, op.stage); break;
         }
     }
+}
+
+// the program's descriptors to `dev`, then its operations; where the descriptors are a kernel parameter, the
+// same launch zeroes the first Memset's range (two launches of 2 us each before)
+int upload_and_issue(oz2_context* h, const Program& prog, unsigned char* dev) {
+    const std::vector<unsigned char>& b = prog.blob;
+    for (const Op& op : prog.ops) {
+        if (op.kind == Op::Mark) continue;
+        if (op.kind != Op::Memset || b.empty() || b.size() > kParamBlobBytes) break;
+        launch_write_blob(b.data(), b.size(), dev, h->stream, op.ptr, op.bytes);
+        ++h->launches;
+        issue(h, prog, dev, &op);
+        return OZ2_OK;
+    }
+    if (int st = put_blob(h, b.data(), b.size(), dev)) return st;
+    issue(h, prog, dev);
+    return OZ2_OK;
 }
 
 // ---------------------------------------------------------------- GEMM configuration
@@ -837,8 +856,7 @@ int run_single(oz2_context* h, const Prob& p) {
     if (prog.blob.size() > align256(desc_bytes_single(L.pm, L.pn)))
         return fail(h, OZ2_EINTERNAL, "oz2: descriptor region too small");
     if ((st = check_grid(h, prog))) return st;
-    if ((st = upload(h, prog, dev_desc))) return st;
-    issue(h, prog, dev_desc);
+    if ((st = upload_and_issue(h, prog, dev_desc))) return st;
     return OZ2_OK;
 }
 
@@ -954,8 +972,7 @@ int run_grouped(oz2_context* h, std::vector<Prob>& probs) {
             h->capturing->execs.push_back(exec);
             OZ2_CUDA(h, cudaGraphLaunch(exec, h->stream));
         } else {
-            if ((st = upload(h, prog, dev_desc))) return st;
-            issue(h, prog, dev_desc);
+            if ((st = upload_and_issue(h, prog, dev_desc))) return st;
         }
     }
     h->tiling[0] = h->tiling[1] = h->tiling[2] = h->tiling[3] = h->tiling[4] = 0;
@@ -1736,7 +1753,7 @@ int run_adaptive(oz2_context* h, std::vector<Prob>& base, const std::vector<int>
             if (obase_desc + prog.blob.size() > h->ws2_size)
                 return fail(h, OZ2_EINTERNAL, "oz2: descriptor region too small");
             if ((st2 = check_grid(h, prog))) return st2;
-            if ((st2 = upload(h, prog, h->ws2 + obase_desc))) return st2;
+            if ((st2 = put_blob(h, prog.blob.data(), prog.blob.size(), h->ws2 + obase_desc))) return st2;
             mark(h, kBegin);
             issue(h, prog, h->ws2 + obase_desc);
         }
@@ -2099,8 +2116,7 @@ int oz2_ozaki1_dgemm(oz2_handle h, int64_t m, int64_t n, int64_t k, const double
     if ((st = check_grid(h, prog))) return st;
     unsigned char* dev_desc = h->ws + o_desc;
     if (prog.blob.size() > (64u << 10)) return fail(h, OZ2_EINTERNAL, "oz2: descriptor region too small");
-    if ((st = upload(h, prog, dev_desc))) return st;
-    issue(h, prog, dev_desc);
+    if ((st = upload_and_issue(h, prog, dev_desc))) return st;
     launch_oz1_horner(acc, m, n, L, maxA, maxB, tk, C, ldc, h->stream);
     ++h->launches;
     return end_call(h, nullptr);

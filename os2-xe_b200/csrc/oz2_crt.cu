@@ -283,17 +283,25 @@ struct alignas(16) BlobParam {
     unsigned char data[N];
     uint32_t bytes;
 };
+// block 0 writes the blob, the others zero their share of [zero, zero + 16 nzero)
 template <int N>
-__global__ void write_blob_kernel(const __grid_constant__ BlobParam<N> b, unsigned char* dst) {
+__global__ void write_blob_kernel(const __grid_constant__ BlobParam<N> b, unsigned char* dst, uint4* zero, size_t nzero) {
+    if (blockIdx.x) {
+        const size_t stride = static_cast<size_t>(gridDim.x - 1) * blockDim.x;
+        for (size_t i = static_cast<size_t>(blockIdx.x - 1) * blockDim.x + threadIdx.x; i < nzero; i += stride)
+            zero[i] = make_uint4(0, 0, 0, 0);
+        return;
+    }
     for (uint32_t i = threadIdx.x * 16; i < b.bytes; i += blockDim.x * 16)
         *reinterpret_cast<uint4*>(dst + i) = *reinterpret_cast<const uint4*>(b.data + i);
 }
 template <int N>
-void write_blob_n(const unsigned char* src, size_t n, unsigned char* dst, cudaStream_t st) {
+void write_blob_n(const unsigned char* src, size_t n, unsigned char* dst, cudaStream_t st, void* zero, size_t zero_bytes) {
     static thread_local BlobParam<N> bp;
     std::memcpy(bp.data, src, n);
     bp.bytes = static_cast<uint32_t>((n + 15) & ~size_t{15});
-    write_blob_kernel<N><<<1, 256, 0, st>>>(bp, dst);
+    const unsigned fill = static_cast<unsigned>(std::min<size_t>((zero_bytes / 16 + 255) / 256, 4 * 148));
+    write_blob_kernel<N><<<1 + fill, 256, 0, st>>>(bp, dst, static_cast<uint4*>(zero), zero_bytes / 16);
 }
 
 // VEC: both pointers 16-byte aligned, 16-byte words first
@@ -449,15 +457,16 @@ void launch_oz1_horner(const int64_t* acc, int64_t m, int64_t n, int L, const un
     oz1_horner_kernel<<<grid, dim3(32, 8), 0, st>>>(acc, m, n, L, maxA, maxB, tk, C, ldc);
 }
 
-void launch_write_blob(const void* src, size_t bytes, void* dst, cudaStream_t st) {
+void launch_write_blob(const void* src, size_t bytes, void* dst, cudaStream_t st, void* zero, size_t zero_bytes) {
     const unsigned char* p = static_cast<const unsigned char*>(src);
     for (size_t off = 0; off < bytes; off += kParamBlobBytes) {
         const size_t n = std::min(kParamBlobBytes, bytes - off);
         unsigned char* d = static_cast<unsigned char*>(dst) + off;
-        if (n <= 1024) write_blob_n<1024>(p + off, n, d, st);
-        else if (n <= 4096) write_blob_n<4096>(p + off, n, d, st);
-        else if (n <= 12288) write_blob_n<12288>(p + off, n, d, st);
-        else write_blob_n<kParamBlobBytes>(p + off, n, d, st);
+        if (n <= 1024) write_blob_n<1024>(p + off, n, d, st, zero, zero_bytes);
+        else if (n <= 4096) write_blob_n<4096>(p + off, n, d, st, zero, zero_bytes);
+        else if (n <= 12288) write_blob_n<12288>(p + off, n, d, st, zero, zero_bytes);
+        else write_blob_n<kParamBlobBytes>(p + off, n, d, st, zero, zero_bytes);
+        zero_bytes = 0;
     }
 }
 

@@ -167,7 +167,8 @@ int64_t crt_item_blocks(CrtItem& it, int64_t block0);
 
 // launches over device tables (d_items) whose host copies (h_items) give the geometry
 void launch_scale(const ScaleItem* d_items, const ScaleItem* h_items, int count, int64_t blocks, cudaStream_t st);
-// all items of one split launch share row_contig, cplx, tc and the narrow/wide/widest limb path;
+// all items of one split launch share cplx, fuse, tc and the narrow/wide/widest limb path, and the layout
+// where fuse or tc is set;
 // err: the device error word for the tensor-core split's bounded wait on its MMA (may be null
 // only for launches without tc items)
 void launch_split(const SplitItem* d_items, const SplitItem* h_items, int count, int64_t blocks, int* err,
@@ -221,9 +222,11 @@ cudaError_t prepare_split_kernels();
 void set_gemm_failure_test(uint64_t wait_ns, int stall);
 
 // Copies up to kParamBlobBytes of host data to device memory by passing them as the parameter
-// of a one-block kernel: no staging buffer, no memcpy, capturable in a graph.
+// of a kernel: no staging buffer, no memcpy, capturable in a graph. The same launch zeroes zero_bytes
+// (a multiple of 16) at `zero` (16-byte aligned).
 constexpr size_t kParamBlobBytes = 30 * 1024;
-void launch_write_blob(const void* src, size_t bytes, void* dst, cudaStream_t st);
+void launch_write_blob(const void* src, size_t bytes, void* dst, cudaStream_t st, void* zero = nullptr,
+                       size_t zero_bytes = 0);
 
 // Copies bytes with SM loads and stores; either side may be pinned host memory, which unified
 // addressing maps into the device's address space. A call moves its own small data (item tables

@@ -42,7 +42,8 @@ __device__ __forceinline__ int find_item(const Item* items, int count, int64_t b
 // ------------------------------------------------------------------ scale
 // ROWC: plane rows contiguous in memory, one thread per row and a k range per block.
 // Otherwise: inner index contiguous, one warp per row and a k range per block.
-template <bool CPLX, bool ROWC>
+// The layout is the item's, so both operands share one launch.
+template <bool CPLX>
 __global__ void __launch_bounds__(256) scale_kernel(const ScaleItem* __restrict__ items, int count) {
     const ScaleItem* I = items + find_item(items, count, blockIdx.x);
     const int64_t local = static_cast<int64_t>(blockIdx.x) - I->block0;
@@ -50,7 +51,7 @@ __global__ void __launch_bounds__(256) scale_kernel(const ScaleItem* __restrict_
     divmod_index(local, I->rblocks, kc, rb);
     const unsigned long long* X = reinterpret_cast<const unsigned long long*>(I->X);
     const int64_t rows = I->rows, k = I->k, ldx = I->ldx, kchunk = I->kchunk;
-    if (ROWC) {
+    if (I->row_contig) {
         // 32 consecutive rows per block (one per lane); the 8 warps interleave the k range
         const int64_t r = rb * 32 + (threadIdx.x & 31);
         if (r >= rows) return;
@@ -470,8 +471,9 @@ __device__ __forceinline__ void split_tiles(const SplitItem* __restrict__ I, Spl
     }
 }
 
-// A block: split_rows rows by I->kspan k blocks; block index -> (row block, k span)
-template <int NW, bool CPLX, bool ROWC>
+// A block: split_rows rows by I->kspan k blocks; block index -> (row block, k span). The layout is the item's
+// (one branch per block), so both operands share one launch.
+template <int NW, bool CPLX>
 __global__ void __launch_bounds__(kSplitThreads, CPLX || NW == 2 ? 2 : 3)
     split_kernel(const SplitItem* __restrict__ items, int count) {
     __shared__ SplitShared<NW> S;
@@ -482,7 +484,8 @@ __global__ void __launch_bounds__(kSplitThreads, CPLX || NW == 2 ? 2 : 3)
     split_consts<NW>(I, S);
     __syncthreads();
     const int kb0 = static_cast<int>(by) * I->kspan, kb1 = min(kb0 + I->kspan, static_cast<int>(I->kb_total));
-    split_tiles<NW, CPLX, ROWC>(I, S, bx * split_rows<CPLX>(), kb0, kb1, I->maxbits, 0);
+    if (I->row_contig) split_tiles<NW, CPLX, true>(I, S, bx * split_rows<CPLX>(), kb0, kb1, I->maxbits, 0);
+    else split_tiles<NW, CPLX, false>(I, S, bx * split_rows<CPLX>(), kb0, kb1, I->maxbits, 0);
 }
 
 // ------------------------------------------------------------------ scale fused into the split
@@ -919,10 +922,8 @@ void scale_split_dispatch(const SplitItem* d, int count, int64_t blocks, bool ro
 }
 
 template <int NW, bool CPLX>
-void split_dispatch(const SplitItem* d, int count, int64_t blocks, bool rowc, cudaStream_t st) {
-    const unsigned g = static_cast<unsigned>(blocks);
-    if (rowc) split_kernel<NW, CPLX, true><<<g, kSplitThreads, 0, st>>>(d, count);
-    else split_kernel<NW, CPLX, false><<<g, kSplitThreads, 0, st>>>(d, count);
+void split_dispatch(const SplitItem* d, int count, int64_t blocks, cudaStream_t st) {
+    split_kernel<NW, CPLX><<<static_cast<unsigned>(blocks), kSplitThreads, 0, st>>>(d, count);
 }
 
 }  // namespace
@@ -1019,15 +1020,9 @@ cudaError_t prepare_split_kernels() {
 
 void launch_scale(const ScaleItem* d, const ScaleItem* h, int count, int64_t blocks, cudaStream_t st) {
     if (count <= 0 || blocks <= 0) return;
-    const bool rowc = h[0].row_contig != 0, cplx = h[0].cplx != 0;
     const unsigned g = static_cast<unsigned>(blocks);
-    if (rowc) {
-        if (cplx) scale_kernel<true, true><<<g, 256, 0, st>>>(d, count);
-        else scale_kernel<false, true><<<g, 256, 0, st>>>(d, count);
-    } else {
-        if (cplx) scale_kernel<true, false><<<g, 256, 0, st>>>(d, count);
-        else scale_kernel<false, false><<<g, 256, 0, st>>>(d, count);
-    }
+    if (h[0].cplx) scale_kernel<true><<<g, 256, 0, st>>>(d, count);
+    else scale_kernel<false><<<g, 256, 0, st>>>(d, count);
 }
 
 void launch_slice(const SplitItem* d, const SplitItem* h, int count, int64_t blocks, cudaStream_t st) {
@@ -1049,12 +1044,12 @@ void launch_split(const SplitItem* d, const SplitItem* h, int count, int64_t blo
         else if (words == 3) split_tc_dispatch<3>(d, count, blocks, rowc, err, st);
         else split_tc_dispatch<2>(d, count, blocks, rowc, err, st);
     } else if (h[0].cplx) {  // s <= 24: at most three words
-        if (words == 3) split_dispatch<3, true>(d, count, blocks, rowc, st);
-        else split_dispatch<2, true>(d, count, blocks, rowc, st);
+        if (words == 3) split_dispatch<3, true>(d, count, blocks, st);
+        else split_dispatch<2, true>(d, count, blocks, st);
     } else {
-        if (words == 4) split_dispatch<4, false>(d, count, blocks, rowc, st);
-        else if (words == 3) split_dispatch<3, false>(d, count, blocks, rowc, st);
-        else split_dispatch<2, false>(d, count, blocks, rowc, st);
+        if (words == 4) split_dispatch<4, false>(d, count, blocks, st);
+        else if (words == 3) split_dispatch<3, false>(d, count, blocks, st);
+        else split_dispatch<2, false>(d, count, blocks, st);
     }
 }
 
