@@ -93,6 +93,7 @@ __global__ void __launch_bounds__(256, CPLX ? 2 : (L <= 8 ? 4 : 3)) crt_kernel(c
     for (int T = 0; T < NT; ++T)
 #pragma unroll
         for (int h = 0; h < KH; ++h) B[T][h] = *reinterpret_cast<const uint32_t*>(&P.wb[8 * T + g][16 * h + 4 * c]);
+    dev::chain_wait();  // no chain_next: what follows is another program's, or the caller's
     int lo = 0, hi = P.count - 1;
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
@@ -258,10 +259,10 @@ void crt_dispatch(int limbs, const CrtParams& P, int64_t blocks, bool cplx, cuda
         const unsigned grid = static_cast<unsigned>(blocks);
         if constexpr (L <= limbs16_for(kMaxModuli))
             if (cplx) {
-                crt_kernel<L, true><<<grid, 256, crt_smem<L, true>(), st>>>(P);
+                launch_chained(crt_kernel<L, true>, grid, 256, crt_smem<L, true>(), st, P);
                 return;
             }
-        crt_kernel<L, false><<<grid, 256, crt_smem<L, false>(), st>>>(P);
+        launch_chained(crt_kernel<L, false>, grid, 256, crt_smem<L, false>(), st, P);
     }
 }
 template <int L>
@@ -286,6 +287,7 @@ struct alignas(16) BlobParam {
 // block 0 writes the blob, the others zero their share of [zero, zero + 16 nzero)
 template <int N>
 __global__ void write_blob_kernel(const __grid_constant__ BlobParam<N> b, unsigned char* dst, uint4* zero, size_t nzero) {
+    dev::chain_next();
     if (blockIdx.x) {
         const size_t stride = static_cast<size_t>(gridDim.x - 1) * blockDim.x;
         for (size_t i = static_cast<size_t>(blockIdx.x - 1) * blockDim.x + threadIdx.x; i < nzero; i += stride)
@@ -321,6 +323,7 @@ __global__ void sm_copy_kernel(const unsigned char* __restrict__ src, unsigned c
 
 template <bool VEC>
 __global__ void fill_kernel(unsigned char* __restrict__ dst, uint32_t word, size_t bytes) {
+    dev::chain_next();
     const size_t tid = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
     size_t tail = 0;

@@ -217,6 +217,9 @@ __global__ void __launch_bounds__(gemm_threads<KIND>(), 1) gemm_i8_modm_kernel(c
     __syncthreads();
     dev::tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    dev::chain_wait();  // barriers and TMEM are ready by now
+    if constexpr (!CRTF) dev::chain_next();
+    asm volatile("fence.proxy.async.global;" ::: "memory");  // the planes were written by ordinary stores
     // The CTA's n-th job for one role: false past the last job, or (ok false) when the wait for its batch ran
     // out; one lane waits (`whole` roles are a warp). job_done(n) releases the batch after its last job.
     constexpr bool SCHED = KIND == kKindQueue;
@@ -631,7 +634,7 @@ GemmParams make_params(const GemmItem* d_items, int count, int group_j, int64_t 
 
 template <int BN, int KIND = kKindResidue>
 void launch_bn(const GemmParams& P, int grid, cudaStream_t st) {
-    gemm_i8_modm_kernel<BN, KIND><<<grid, gemm_threads<KIND>(), gemm_smem<BN, KIND>(), st>>>(P);
+    launch_chained(gemm_i8_modm_kernel<BN, KIND>, static_cast<unsigned>(grid), gemm_threads<KIND>(), gemm_smem<BN, KIND>(), st, P);
 }
 
 }  // namespace

@@ -165,6 +165,25 @@ bool fuse_scale(bool cplx, bool row_contig, int64_t k);
 void crt_launch_shape(CrtItem* items, int count, const Plan& plan, bool cplx);
 int64_t crt_item_blocks(CrtItem& it, int64_t block0);
 
+// A launch that may start while the kernel before it on the stream still runs: its blocks are placed as that
+// one's drain and wait in dev::chain_wait(), so the launch latency and the prologue are hidden. Only for kernels
+// that call chain_wait() in every block before their first global access; the completion of each then implies
+// the completion of all before it, so a later plain launch, copy or event sees them all.
+template <class... P, class... A>
+void launch_chained(void (*kernel)(P...), unsigned grid, unsigned threads, size_t smem, cudaStream_t st, A... args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // launches over device tables (d_items) whose host copies (h_items) give the geometry
 void launch_scale(const ScaleItem* d_items, const ScaleItem* h_items, int count, int64_t blocks, cudaStream_t st);
 // all items of one split launch share cplx, fuse, tc and the narrow/wide/widest limb path, and the layout

@@ -8,6 +8,12 @@
 namespace oz2 {
 namespace dev {
 
+// Programmatic dependent launch (launch_chained): a kernel of a chain waits here, before its first global
+// access, until every kernel before it has finished and its writes are visible, then lets the next one's
+// blocks start (theirs wait in turn). No-ops in a kernel launched without the attribute.
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // Device-side error codes written to the handle's error word (host maps them to OZ2_ETIMEOUT).
 enum : int { kErrNone = 0, kErrTimeoutFull = 1, kErrTimeoutEmpty = 2, kErrTimeoutAccFull = 3,
              kErrTimeoutAccEmpty = 4, kErrTimeoutDrain = 5, kErrTimeoutJobs = 6 };

@@ -45,6 +45,8 @@ __device__ __forceinline__ int find_item(const Item* items, int count, int64_t b
 // The layout is the item's, so both operands share one launch.
 template <bool CPLX>
 __global__ void __launch_bounds__(256) scale_kernel(const ScaleItem* __restrict__ items, int count) {
+    dev::chain_wait();
+    dev::chain_next();
     const ScaleItem* I = items + find_item(items, count, blockIdx.x);
     const int64_t local = static_cast<int64_t>(blockIdx.x) - I->block0;
     int64_t rb, kc;
@@ -477,6 +479,9 @@ template <int NW, bool CPLX>
 __global__ void __launch_bounds__(kSplitThreads, CPLX || NW == 2 ? 2 : 3)
     split_kernel(const SplitItem* __restrict__ items, int count) {
     __shared__ SplitShared<NW> S;
+    // no chain_next: GEMM blocks placed while these drain land on the SMs in the order they fall free, and tiles
+    // that share operands drift apart (8192^3, s = 14: 7.75 ms, 8.3 ms so placed)
+    dev::chain_wait();
     const SplitItem* __restrict__ I = items + find_item(items, count, blockIdx.x);
     const int64_t local = static_cast<int64_t>(blockIdx.x) - I->block0;
     int64_t bx, by;
@@ -923,7 +928,7 @@ void scale_split_dispatch(const SplitItem* d, int count, int64_t blocks, bool ro
 
 template <int NW, bool CPLX>
 void split_dispatch(const SplitItem* d, int count, int64_t blocks, cudaStream_t st) {
-    split_kernel<NW, CPLX><<<static_cast<unsigned>(blocks), kSplitThreads, 0, st>>>(d, count);
+    launch_chained(split_kernel<NW, CPLX>, static_cast<unsigned>(blocks), kSplitThreads, 0, st, d, count);
 }
 
 }  // namespace
@@ -1021,8 +1026,8 @@ cudaError_t prepare_split_kernels() {
 void launch_scale(const ScaleItem* d, const ScaleItem* h, int count, int64_t blocks, cudaStream_t st) {
     if (count <= 0 || blocks <= 0) return;
     const unsigned g = static_cast<unsigned>(blocks);
-    if (h[0].cplx) scale_kernel<true><<<g, 256, 0, st>>>(d, count);
-    else scale_kernel<false><<<g, 256, 0, st>>>(d, count);
+    if (h[0].cplx) launch_chained(scale_kernel<true>, g, 256, 0, st, d, count);
+    else launch_chained(scale_kernel<false>, g, 256, 0, st, d, count);
 }
 
 void launch_slice(const SplitItem* d, const SplitItem* h, int count, int64_t blocks, cudaStream_t st) {

@@ -1,0 +1,56 @@
+"""Launches that share operands of both layouts and start while the one before drains: chains of products that
+read the previous result at once, on the default and on a side stream, and grouped calls with every op pair
+(descriptors as a kernel parameter and through the staging ring), bit for bit against the oracle."""
+import numpy as np
+import pytest
+
+from common import bits, from_dev, make_mat, to_dev
+
+pytestmark = pytest.mark.gpu
+OPS = ("NN", "NT", "TN", "TT")
+
+
+@pytest.mark.parametrize("side", [False, True])
+@pytest.mark.parametrize("n,s", [(1, 14), (40, 6), (129, 16), (260, 20)])
+def test_chain(oracle, oz, n, s, side):
+    import torch
+    A, B = make_mat(1, n, n, n, "u"), make_mat(2, n, n, n, "u")
+    dA, dB, outs = to_dev(A), to_dev(B), [to_dev(np.zeros((n, n), order="F")) for _ in range(6)]
+    torch.cuda.synchronize()
+    st = torch.cuda.Stream() if side else None
+    if side:
+        oz.set_stream(st.cuda_stream)
+    try:
+        for i, out in enumerate(outs):
+            src, op = (outs[i - 1] if i else dA), OPS[i % 4]
+            oz.gemm(op[0], op[1], n, n, n, 1.0, src, n, dB, n, 0.0, out, n, s)
+        torch.cuda.synchronize()
+    finally:
+        if side:
+            oz.set_stream(0)
+    x = A
+    for i, out in enumerate(outs):
+        want, op = np.zeros((n, n), order="F"), OPS[i % 4]
+        assert oracle.dgemm(op[0], op[1], n, n, n, 1.0, x, n, B, n, 0.0, want, n, s) == 0
+        assert np.array_equal(bits(from_dev(out, want)), bits(want)), i
+        x = want
+
+
+@pytest.mark.parametrize("copies", [1, 24])
+def test_grouped_layouts(oracle, oz, copies):
+    import torch
+    probs, keep = [], []
+    for i in range(8 * copies):
+        m, n, k, s, op = 30 + i % 8 * 17, 140 - i % 8 * 13, 1 + i % 8 * 37, (8, 14, 20)[i % 3], OPS[i % 4]
+        sa, sb = ((m, k) if op[0] == "N" else (k, m)), ((k, n) if op[1] == "N" else (n, k))
+        A, B = make_mat(i, sa[0], sa[1], sa[0], "u"), make_mat(i + 99, sb[0], sb[1], sb[0], "u")
+        C = np.zeros((m, n), order="F")
+        dC = to_dev(C)
+        probs.append((op[0], op[1], m, n, k, 1.0, to_dev(A), sa[0], to_dev(B), sb[0], 0.0, dC, m, s))
+        keep.append((A, B, C, dC))
+    oz.gemm_grouped(probs)
+    torch.cuda.synchronize()
+    for p, (A, B, C, dC) in zip(probs, keep):
+        want = C.copy(order="F")
+        assert oracle.dgemm(p[0], p[1], p[2], p[3], p[4], 1.0, A, p[7], B, p[9], 0.0, want, p[2], p[13]) == 0
+        assert np.array_equal(bits(from_dev(dC, C)), bits(want)), p[:5]
