@@ -1324,7 +1324,7 @@ int run_adaptive(oz2_context* h, std::vector<Prob>& base, const std::vector<int>
     ++h->launches;
 
     Program ph1;
-    // with every k up to kFusedStatsMaxK one launch per layout takes the row maxima and the panel
+    // with every k up to kFusedStatsMaxK one launch takes the row maxima and the panel
     // statistics together (one read of A and B from DRAM); otherwise the scale pass runs first
     int64_t kmax = 0;
     for (const Prob& p : base) kmax = std::max(kmax, p.k);
@@ -1335,7 +1335,8 @@ int run_adaptive(oz2_context* h, std::vector<Prob>& base, const std::vector<int>
         sc.push_back(scale_item(base[q], false, maxB(static_cast<int>(q))));
     }
     plan_scale(h, ph1, sc);
-    // panel statistics, grouped by layout
+    // panel statistics, grouped by layout; the fused pass takes both in one launch, the layout with rows
+    // contiguous (32 rows per block, 8 in the other) first
     std::map<int, std::vector<StatItem>> stat_groups;
     for (size_t q = 0; q < base.size(); ++q) {
         const Prob& p = base[q];
@@ -1353,7 +1354,7 @@ int run_adaptive(oz2_context* h, std::vector<Prob>& base, const std::vector<int>
                 it.row_contig = rowc;
                 it.maxbits = (side ? maxB(static_cast<int>(q)) : maxA(static_cast<int>(q))) + r0;
                 it.hist = hist((side ? pb0[q] : pa0[q]) + pi);
-                stat_groups[rowc].push_back(it);
+                stat_groups[fused_stats ? 0 : rowc].push_back(it);
             }
         }
     }
@@ -1364,6 +1365,8 @@ int run_adaptive(oz2_context* h, std::vector<Prob>& base, const std::vector<int>
     };
     std::vector<StatOp> stat_ops;
     for (auto& kv : stat_groups) {
+        if (fused_stats)
+            std::stable_partition(kv.second.begin(), kv.second.end(), [](const StatItem& it) { return it.row_contig != 0; });
         int64_t blocks = 0;
         for (auto& it : kv.second)
             blocks += fused_stats ? scale_stat_item_blocks(it, blocks) : stat_item_blocks(it, blocks);
@@ -1401,7 +1404,7 @@ int run_adaptive(oz2_context* h, std::vector<Prob>& base, const std::vector<int>
     for (const StatOp& so : stat_ops) {
         const StatItem* d_items = reinterpret_cast<const StatItem*>(dd + so.off);
         const StatItem* h_items = reinterpret_cast<const StatItem*>(ph1.blob.data() + so.off);
-        if (fused_stats) launch_scale_stats(d_items, h_items, so.count, so.blocks, h->stream);
+        if (fused_stats) launch_scale_stats(d_items, so.count, so.blocks, h->stream);
         else launch_panel_stats(d_items, h_items, so.count, so.blocks, h->stream);
         ++h->launches;
     }
