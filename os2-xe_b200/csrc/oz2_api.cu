@@ -50,6 +50,7 @@ struct Op {
     int64_t m = 0, n = 0, ldc = 0;  // scale_c
     double beta[2] = {0, 0};
     int stage = 0;
+    bool first = false;  // scale: launch_scale_first
 };
 
 struct Program {
@@ -529,14 +530,18 @@ void plan_tasks(Program& prog, const std::vector<Task>& tasks, const GemmConfig&
     prog.ops.push_back(mk);
 }
 
-void plan_scale(oz2_context* h, Program& prog, std::vector<ScaleItem>& items) {
+// `first`: the items are the whole of a small program's scale pass, which its first launch takes (upload_and_issue)
+void plan_scale(oz2_context* h, Program& prog, std::vector<ScaleItem>& items, bool first = false) {
     std::map<int, std::vector<ScaleItem>> groups;  // real, complex
     for (auto& it : items) groups[it.cplx].push_back(it);
     for (auto& kv : groups) {
         int64_t blocks = 0;
-        for (auto& it : kv.second) blocks += scale_item_blocks(it, h->num_sms, blocks);
+        for (auto& it : kv.second)
+            blocks += first ? scale_rows_blocks(it, blocks) : scale_item_blocks(it, h->num_sms, blocks);
         Op op;
         op.kind = Op::Scale;
+        op.first = first;
+        op.cplx = kv.first != 0;
         op.count = static_cast<int>(kv.second.size());
         op.blocks = blocks;
         op.off = prog.add(kv.second.data(), kv.second.size() * sizeof(ScaleItem));
@@ -644,11 +649,11 @@ int read_back(oz2_context* h, std::initializer_list<HostRead> reads) {
     return OZ2_OK;
 }
 
-// `filled`: a Memset that the launch before this one made
-void issue(oz2_context* h, const Program& prog, const unsigned char* dev, const Op* filled = nullptr) {
+// the operations from index `from` on
+void issue(oz2_context* h, const Program& prog, const unsigned char* dev, size_t from = 0) {
     const unsigned char* hb = prog.blob.data();
-    for (const Op& op : prog.ops) {
-        if (&op == filled) continue;
+    for (size_t q = from; q < prog.ops.size(); ++q) {
+        const Op& op = prog.ops[q];
         if (op.kind != Op::Mark) ++h->launches;
         switch (op.kind) {
             case Op::Memset: launch_fill(op.ptr, 0, op.bytes, h->stream); break;
@@ -686,19 +691,28 @@ void issue(oz2_context* h, const Program& prog, const unsigned char* dev, const 
 }
 
 // the program's descriptors to `dev`, then its operations; where the descriptors are a kernel parameter, the
-// same launch zeroes the first Memset's range (two launches of 2 us each before)
+// same launch takes a small program's scale pass, or zeroes the first Memset's range
 int upload_and_issue(oz2_context* h, const Program& prog, unsigned char* dev) {
     const std::vector<unsigned char>& b = prog.blob;
-    for (const Op& op : prog.ops) {
-        if (op.kind == Op::Mark) continue;
-        if (op.kind != Op::Memset || b.empty() || b.size() > kParamBlobBytes) break;
-        launch_write_blob(b.data(), b.size(), dev, h->stream, op.ptr, op.bytes);
-        ++h->launches;
-        issue(h, prog, dev, &op);
+    size_t q = 0;
+    while (q < prog.ops.size() && prog.ops[q].kind == Op::Mark) ++q;
+    const bool first = q < prog.ops.size() && prog.ops[q].first;
+    const bool zero = q < prog.ops.size() && prog.ops[q].kind == Op::Memset && !b.empty() && b.size() <= kParamBlobBytes;
+    if (!first && !zero) {
+        if (int st = put_blob(h, b.data(), b.size(), dev)) return st;
+        issue(h, prog, dev);
         return OZ2_OK;
     }
-    if (int st = put_blob(h, b.data(), b.size(), dev)) return st;
-    issue(h, prog, dev);
+    const Op& op = prog.ops[q];
+    if (first) {  // run_single keeps such a program below kScaleFirstBytes; the launch belongs to the scale stage
+        for (size_t i = 0; i < q; ++i) mark(h, prog.ops[i].stage);
+        launch_scale_first(b.data(), b.size(), dev, op.off, op.count, op.blocks, op.cplx, h->stream);
+    } else {
+        launch_write_blob(b.data(), b.size(), dev, h->stream, op.ptr, op.bytes);
+        for (size_t i = 0; i < q; ++i) mark(h, prog.ops[i].stage);
+    }
+    ++h->launches;
+    issue(h, prog, dev, q + 1);
     return OZ2_OK;
 }
 
@@ -835,16 +849,20 @@ int run_single(oz2_context* h, const Prob& p) {
     mk.kind = Op::Mark;
     mk.stage = kBegin;
     prog.ops.push_back(mk);
-    Op ms;
-    ms.kind = Op::Memset;
-    ms.ptr = maxA;
-    ms.bytes = reinterpret_cast<unsigned char*>(planesA) - reinterpret_cast<unsigned char*>(maxA);
-    prog.ops.push_back(ms);
     const bool fa = fuse_side(p, true), fb = fuse_side(p, false);
+    // one tile: its seven descriptors stay below kScaleFirstBytes
+    const bool first = !fa && !fb && L.pm == 1 && L.pn == 1 && p.k > 0 && p.k * (p.G == 3 ? 2 : 1) <= kScaleFirstMaxK;
+    if (!first) {
+        Op ms;
+        ms.kind = Op::Memset;
+        ms.ptr = maxA;
+        ms.bytes = reinterpret_cast<unsigned char*>(planesA) - reinterpret_cast<unsigned char*>(maxA);
+        prog.ops.push_back(ms);
+    }
     std::vector<ScaleItem> sc;
     if (!fa) sc.push_back(scale_item(p, true, maxA));
     if (!fb) sc.push_back(scale_item(p, false, maxB));
-    plan_scale(h, prog, sc);
+    plan_scale(h, prog, sc, first);
     const int64_t ldr = round_up(L.mb, 32);
     for (int64_t j0 = 0; j0 < p.n; j0 += L.nb) {
         for (int64_t i0 = 0; i0 < p.m; i0 += L.mb) {
@@ -853,7 +871,7 @@ int run_single(oz2_context* h, const Prob& p) {
             plan_tasks(prog, {t}, cfg);
         }
     }
-    if (prog.blob.size() > align256(desc_bytes_single(L.pm, L.pn)))
+    if (prog.blob.size() > align256(desc_bytes_single(L.pm, L.pn)) || (first && prog.blob.size() > kScaleFirstBytes))
         return fail(h, OZ2_EINTERNAL, "oz2: descriptor region too small");
     if ((st = check_grid(h, prog))) return st;
     if ((st = upload_and_issue(h, prog, dev_desc))) return st;

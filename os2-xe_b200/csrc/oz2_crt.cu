@@ -278,12 +278,6 @@ cudaError_t crt_prepare() {
     }
 }
 
-// the parameter block is copied with every launch: size classes keep small blobs cheap
-template <int N>
-struct alignas(16) BlobParam {
-    unsigned char data[N];
-    uint32_t bytes;
-};
 // block 0 writes the blob, the others zero their share of [zero, zero + 16 nzero)
 template <int N>
 __global__ void write_blob_kernel(const __grid_constant__ BlobParam<N> b, unsigned char* dst, uint4* zero, size_t nzero) {

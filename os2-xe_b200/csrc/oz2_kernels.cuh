@@ -184,6 +184,14 @@ void launch_chained(void (*kernel)(P...), unsigned grid, unsigned threads, size_
     cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
+// the scale pass of a program that fits kScaleFirstBytes, in the launch that writes its descriptors: whole rows per
+// block, so their maxima need no zeroing (items as scale_rows_blocks laid them out, at `off` in the program)
+constexpr int64_t kScaleFirstMaxK = 512;
+constexpr size_t kScaleFirstBytes = 12288;
+int64_t scale_rows_blocks(ScaleItem& it, int64_t block0);
+void launch_scale_first(const void* blob, size_t bytes, void* dst, size_t off, int count, int64_t blocks, bool cplx,
+                        cudaStream_t st);
+
 // launches over device tables (d_items) whose host copies (h_items) give the geometry
 void launch_scale(const ScaleItem* d_items, const ScaleItem* h_items, int count, int64_t blocks, cudaStream_t st);
 // all items of one split launch share cplx, fuse, tc and the narrow/wide/widest limb path, and the layout
@@ -239,6 +247,13 @@ cudaError_t prepare_split_kernels();
 // issues nothing, so the other roles' waits run out, record their code in the error word, drain
 // their copies, free TMEM and return.
 void set_gemm_failure_test(uint64_t wait_ns, int stall);
+
+// the parameter block is copied with every launch: size classes keep small blobs cheap
+template <int N>
+struct alignas(16) BlobParam {
+    unsigned char data[N];
+    uint32_t bytes;
+};
 
 // Copies up to kParamBlobBytes of host data to device memory by passing them as the parameter
 // of a kernel: no staging buffer, no memcpy, capturable in a graph. The same launch zeroes zero_bytes

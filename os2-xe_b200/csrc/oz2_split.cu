@@ -9,6 +9,7 @@
 //        stored as int8 in the pre-tiled plane layout of oz2_kernels.cuh.
 #include <algorithm>
 #include <atomic>
+#include <cstring>
 
 #include "oz2_kernels.cuh"
 #include "oz2_ptx.cuh"
@@ -82,6 +83,62 @@ __global__ void __launch_bounds__(256) scale_kernel(const ScaleItem* __restrict_
         for (int o = 16; o > 0; o >>= 1) best = max(best, __shfl_xor_sync(0xFFFFFFFFu, best, o));
         if (lane == 0 && best) atomicMax(I->out + r, best);
     }
+}
+
+// The same maxima as the first launch of a small product: the descriptors come as the kernel's parameter, the last
+// block writes them for the kernels that follow, and a block owns 32 whole rows (rows contiguous: a lane per row, 32
+// warps interleave k; otherwise a warp per row), so its stores need no zeroed maxima. For k <= kScaleFirstMaxK, where
+// a thread reads at most 16 entries, eight in flight: 256^3 24.0 -> 20.4 us per call back to back, 1024 x 1024 x 512
+// 41.2 -> 37.3; at k = 1024 the few blocks take longer than the launch saved (1024^3 57 -> 64 us), splitting k wins.
+template <int N, bool CPLX>
+__global__ void __launch_bounds__(1024) scale_first_kernel(const __grid_constant__ BlobParam<N> b, unsigned char* dst,
+                                                           uint32_t off, int count) {
+    __shared__ unsigned long long part[32][33];
+    dev::chain_next();
+    if (blockIdx.x == gridDim.x - 1) {
+        for (uint32_t i = threadIdx.x * 16; i < b.bytes; i += 1024 * 16)
+            *reinterpret_cast<uint4*>(dst + i) = *reinterpret_cast<const uint4*>(b.data + i);
+        return;
+    }
+    const ScaleItem* items = reinterpret_cast<const ScaleItem*>(b.data + off);
+    const ScaleItem* I = items + find_item(items, count, blockIdx.x);
+    const int64_t r0 = (static_cast<int64_t>(blockIdx.x) - I->block0) * 32;
+    const int warp = static_cast<int>(threadIdx.x >> 5), lane = static_cast<int>(threadIdx.x & 31);
+    constexpr int W = CPLX ? 2 : 1;
+    const unsigned long long* X = reinterpret_cast<const unsigned long long*>(I->X);
+    const int k = static_cast<int>(I->k);
+    unsigned long long best = 0;
+    if (I->row_contig) {
+        const int64_t r = r0 + lane, ldx = I->ldx;
+        if (r < I->rows) {
+#pragma unroll 8
+            for (int p = warp; p < k; p += 32) {
+                const unsigned long long* x = X + W * (r + p * ldx);
+                best = max(best, __ldg(x) & kAbsMask);
+                if (CPLX) best = max(best, __ldg(x + 1) & kAbsMask);
+            }
+        }
+        part[lane][warp] = best;
+        __syncthreads();
+        best = part[warp][lane];
+    } else if (r0 + warp < I->rows) {
+        const unsigned long long* x = X + W * (r0 + warp) * I->ldx;
+#pragma unroll 8
+        for (int p = lane; p < W * k; p += 32) best = max(best, __ldg(x + p) & kAbsMask);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) best = max(best, __shfl_xor_sync(0xFFFFFFFFu, best, o));
+    if (lane == 0 && r0 + warp < I->rows) I->out[r0 + warp] = best;
+}
+
+template <int N>
+void scale_first_n(const void* blob, size_t bytes, unsigned char* dst, uint32_t off, int count, unsigned grid, bool cplx,
+                   cudaStream_t st) {
+    static thread_local BlobParam<N> bp;
+    std::memcpy(bp.data, blob, bytes);
+    bp.bytes = static_cast<uint32_t>((bytes + 15) & ~size_t{15});
+    if (cplx) scale_first_kernel<N, true><<<grid, 1024, 0, st>>>(bp, dst, off, count);
+    else scale_first_kernel<N, false><<<grid, 1024, 0, st>>>(bp, dst, off, count);
 }
 
 // ------------------------------------------------------------------ split
@@ -1028,6 +1085,22 @@ void launch_scale(const ScaleItem* d, const ScaleItem* h, int count, int64_t blo
     const unsigned g = static_cast<unsigned>(blocks);
     if (h[0].cplx) launch_chained(scale_kernel<true>, g, 256, 0, st, d, count);
     else launch_chained(scale_kernel<false>, g, 256, 0, st, d, count);
+}
+
+int64_t scale_rows_blocks(ScaleItem& it, int64_t block0) {
+    it.block0 = block0;
+    it.rblocks = ceil_div(it.rows, 32);
+    it.kchunk = it.k;
+    return it.rblocks;
+}
+
+void launch_scale_first(const void* blob, size_t bytes, void* dst, size_t off, int count, int64_t blocks, bool cplx,
+                        cudaStream_t st) {
+    unsigned char* d = static_cast<unsigned char*>(dst);
+    const unsigned grid = static_cast<unsigned>(blocks) + 1;
+    const uint32_t o = static_cast<uint32_t>(off);
+    if (bytes <= 4608) scale_first_n<4608>(blob, bytes, d, o, count, grid, cplx, st);  // two operands: 4248
+    else scale_first_n<kScaleFirstBytes>(blob, bytes, d, o, count, grid, cplx, st);
 }
 
 void launch_slice(const SplitItem* d, const SplitItem* h, int count, int64_t blocks, cudaStream_t st) {

@@ -54,3 +54,22 @@ def test_grouped_layouts(oracle, oz, copies):
         want = C.copy(order="F")
         assert oracle.dgemm(p[0], p[1], p[2], p[3], p[4], 1.0, A, p[7], B, p[9], 0.0, want, p[2], p[13]) == 0
         assert np.array_equal(bits(from_dev(dC, C)), bits(want)), p[:5]
+
+
+@pytest.mark.parametrize("op", OPS)
+@pytest.mark.parametrize("m,n,k", [(1, 1, 1), (31, 33, 31), (32, 64, 32), (33, 31, 33), (65, 40, 511), (40, 65, 512),
+                                   (33, 33, 513)])
+def test_first_launch(oracle, oz, m, n, k, op):
+    """the scale pass in the first launch (k up to 512) and beyond it, padded leading dimensions, a zero row"""
+    import torch
+    sa, sb = ((m, k) if op[0] == "N" else (k, m)), ((k, n) if op[1] == "N" else (n, k))
+    la, lb = sa[0] + 3, sb[0] + 1
+    A, B = make_mat(m, sa[0], sa[1], la, "u"), make_mat(n, sb[0], sb[1], lb, "u")
+    A[sa[0] // 2, :] = 0.0
+    C = make_mat(5, m, n, m, "u")
+    dC = to_dev(C)
+    oz.gemm(op[0], op[1], m, n, k, 1.5, to_dev(A), la, to_dev(B), lb, -0.5, dC, m, 15)
+    torch.cuda.synchronize()
+    want = C.copy(order="F")
+    assert oracle.dgemm(op[0], op[1], m, n, k, 1.5, A, la, B, lb, -0.5, want, m, 15) == 0
+    assert np.array_equal(bits(from_dev(dC, C)), bits(want))
