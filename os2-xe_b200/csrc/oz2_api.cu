@@ -1434,6 +1434,20 @@ int run_adaptive(oz2_context* h, std::vector<Prob>& base, const std::vector<int>
         launch_mlp_infer(h->d_mlp, static_cast<int>(ntiles), d_feat, h->mlp_threshold, d_sm, nullptr, h->stream);
         ++h->launches;
     }
+    // What the tile workspace may grow to: the first workspace holds phase-1 data, the second may use what is left.
+    // Asked for while the device takes the statistics: the query takes 0.1 to 3 ms, and between the phases the
+    // device waited for it.
+    size_t tile_limit = h->ws_limit;
+    if (!tile_limit && mode >= 0) {
+        size_t free_b = 0, total = 0;
+        if (cudaMemGetInfo(&free_b, &total) != cudaSuccess) return fail(h, OZ2_ECUDA, "oz2: cudaMemGetInfo");
+        free_b += h->ws2_size;
+        const size_t reserve = (size_t{512} << 20) + total / 32;
+        tile_limit = free_b > reserve ? free_b - reserve : 0;
+        // a batch of 16 GiB of planes and residues keeps every SM busy for milliseconds; more
+        // only takes memory from the rest of the process (the caller's tensors, other calls)
+        tile_limit = std::min(tile_limit, size_t{16} << 30);
+    }
     constexpr int kNoCertificate = 0x7F7F7F7F;  // the device's fill byte 0x7F: above every s
     std::vector<int> s_an(ntiles), s_ml(ntiles, kMaxModuli), s_ce(ntiles, kNoCertificate);
     const size_t tile_bytes = static_cast<size_t>(ntiles) * 4;
@@ -1634,18 +1648,7 @@ int run_adaptive(oz2_context* h, std::vector<Prob>& base, const std::vector<int>
             prob_for[key] = raw;
             return raw;
         };
-        // the first workspace holds phase-1 data; the second may use what is left
-        size_t limit = h->ws_limit;
-        if (!limit) {
-            size_t free_b = 0, total = 0;
-            if (cudaMemGetInfo(&free_b, &total) != cudaSuccess) return fail(h, OZ2_ECUDA, "oz2: cudaMemGetInfo");
-            free_b += h->ws2_size;
-            const size_t reserve = (size_t{512} << 20) + total / 32;
-            limit = free_b > reserve ? free_b - reserve : 0;
-            // a batch of 16 GiB of planes and residues keeps every SM busy for milliseconds; more
-            // only takes memory from the rest of the process (the caller's tensors, other calls)
-            limit = std::min(limit, size_t{16} << 30);
-        }
+        const size_t limit = tile_limit;
         // a problem whose tiles all run here at one s is one task: its GEMM jobs then share the
         // planes through the L2 across the whole problem, as in a plain call
         struct Unit {
