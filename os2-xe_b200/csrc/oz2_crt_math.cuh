@@ -104,14 +104,27 @@ __device__ __forceinline__ double crt_round(const uint32_t (&w)[(L + 1) / 2], in
     uint32_t m = word(1), l = low(2);
     int E = 16 * L - 96 - shift;
     if (w[0] + 1u <= 1u) {  // h is 0 or -1: x is small beside M
+        if constexpr (NW > 1) {
+            // past the words that only repeat the sign, by selects, as lanes differ in how many they have (a branch and
+            // a double per word before: 6144^2 wide entries, s = 20, 560 -> 537 us; 4096^2, s = 24, 236 -> 227)
+            uint32_t v[NW];
 #pragma unroll
-        for (int k = 1; k < NW; ++k)
-            if (dt == 0.0 || dt == -1.0) {
-                dt = __fma_rn(dt, 4294967296.0, u32_double(w[k]));
-                m = word(k + 1);
-                l = low(k + 2);
-                E -= 32;
+            for (int i = 0; i < NW; ++i) v[i] = word(i + 1);
+            E -= 32;
+#pragma unroll
+            for (int k = 2; k < NW; ++k) {
+                const bool skip = v[0] == w[0];
+#pragma unroll
+                for (int i = 0; i + 1 < NW; ++i) v[i] = skip ? v[i + 1] : v[i];
+                E -= skip ? 32 : 0;
             }
+            uint32_t rest = 0;
+#pragma unroll
+            for (int i = 3; i < NW; ++i) rest |= v[i];
+            dt = __fma_rn(dt, 4294967296.0, u32_double(v[0]));
+            m = v[1];
+            l = (NW > 2 ? v[NW > 2 ? 2 : 0] : 0u) | (rest != 0 ? 1u : 0u);
+        }
         if (dt == 0.0) return shift >= kFarExponent / 2 ? __longlong_as_double(0x7FF8000000000000ll) : 0.0;
     }
     // |dt| 2^32 > m, so the first sum's error is exact; (e 2^32 + l) is below 2^45 and exact; the
