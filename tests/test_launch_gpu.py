@@ -73,3 +73,31 @@ def test_first_launch(oracle, oz, m, n, k, op):
     want = C.copy(order="F")
     assert oracle.dgemm(op[0], op[1], m, n, k, 1.5, A, la, B, lb, -0.5, want, m, 15) == 0
     assert np.array_equal(bits(from_dev(dC, C)), bits(want))
+
+
+@pytest.mark.parametrize("k", [300, 700])
+def test_user_capture(oracle, oz, k):
+    """a product captured by the caller into a CUDA graph (chained launches become graph edges), replayed on new data"""
+    import torch
+    m, n, s = 150, 90, 14
+    dA, dB, dC = to_dev(np.zeros((m, k), order="F")), to_dev(np.zeros((k, n), order="F")), to_dev(np.zeros((m, n), order="F"))
+    st = torch.cuda.Stream()
+    oz.set_stream(st.cuda_stream)
+    try:
+        oz.gemm("N", "N", m, n, k, 1.0, dA, m, dB, k, 0.0, dC, m, s)  # the workspace grows outside the capture
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=st):
+            oz.gemm("N", "N", m, n, k, 1.0, dA, m, dB, k, 0.0, dC, m, s)
+        for seed in (1, 2):
+            A, B = make_mat(seed, m, k, m, "u"), make_mat(seed + 7, k, n, k, "u")
+            dA.copy_(to_dev(A))
+            dB.copy_(to_dev(B))
+            g.replay()
+            torch.cuda.synchronize()
+            want = np.zeros((m, n), order="F")
+            assert oracle.dgemm("N", "N", m, n, k, 1.0, A, m, B, k, 0.0, want, m, s) == 0
+            assert np.array_equal(bits(from_dev(dC, want)), bits(want))
+    finally:
+        torch.cuda.synchronize()
+        oz.set_stream(0)
