@@ -92,20 +92,25 @@ int64_t inverse_mod(int64_t a, int64_t m) {
 }
 
 uint32_t pow2_mod(int e, uint32_t m) {
-    uint32_t v = 1 % m;
-    for (int i = 0; i < e; ++i) v = (v * 2) % m;
-    return v;
+    uint64_t v = 1 % m;
+    for (; e > 32; e -= 32) v = (v << 32) % m;
+    return static_cast<uint32_t>((v << e) % m);
 }
 
 }  // namespace
 
 namespace {
-// everything of a plan but tk depends on s alone: built once per s
+// everything of a plan but tk and the split's constants, which follow from tk's number of words, depends on s
+// alone: built once per s (the planning calls make a plan per s they try)
 struct Templates {
     Plan plan[kMaxModuliExt + 1];
+    SplitMod split[kMaxModuliExt + 1][3][kMaxModuliExt];  // for two, three, four words
     int status[kMaxModuliExt + 1];
     Templates() {
-        for (int s = 2; s <= kMaxModuliExt; ++s) status[s] = build(s, plan[s]);
+        for (int s = 2; s <= kMaxModuliExt; ++s) {
+            status[s] = build(s, plan[s]);
+            for (int words = 2; words <= 4 && status[s] == 0; ++words) split_constants(plan[s], words, split[s][words - 2]);
+        }
     }
     static int build(int s, Plan& p) {
         p = Plan{};
@@ -193,7 +198,7 @@ int make_plan_ext(int s, int64_t k, Plan& p) {
     if (tk > (s <= kMaxModuli ? kWideScaleBits : kMaxScaleBitsExt)) return 5;
     p = T.plan[s];
     p.tk = tk;
-    split_constants(p, p.sm);
+    std::memcpy(p.sm, T.split[s][split_words(tk) - 2], s * sizeof(SplitMod));
     return 0;
 }
 
@@ -240,8 +245,8 @@ void mod_constants(const Plan& p, ModConst* out) {
     }
 }
 
-void split_constants(const Plan& p, SplitMod* out) {
-    const int words = split_words(p.tk), top = words == 2 ? 62 : (words == 3 ? 93 : 125);
+void split_constants(const Plan& p, int words, SplitMod* out) {
+    const int top = words == 2 ? 62 : (words == 3 ? 93 : 125);
     for (int t = 0; t < p.s; ++t) {
         const uint32_t m = p.m[t];
         SplitMod& c = out[t];

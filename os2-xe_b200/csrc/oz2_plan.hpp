@@ -94,7 +94,7 @@ struct Plan {
     uint32_t W[kMaxModuliExt][kBigWords] = {};  // CRT weights (M/m_t) y_t
     uint32_t M[kBigWords] = {};
     ModConst mc[kMaxModuliExt] = {};            // the GEMM's per-modulus constants (mod_constants)
-    SplitMod sm[kMaxModuliExt] = {};            // the split's (split_constants, for this tk)
+    SplitMod sm[kMaxModuliExt] = {};            // the split's (split_constants, for the words of this tk)
 };
 
 // Returns 0, or 1 (invalid: s out of [2, 24], k < 1, s too small for k), or 5 (overflow).
@@ -112,7 +112,8 @@ int plan_tk(int s, int64_t k);
 const char* plan_error_text(int s, int64_t k, int status, char* buf, int len);
 
 void mod_constants(const Plan& p, ModConst* out);
-void split_constants(const Plan& p, SplitMod* out);
+// for offset integers of `words` 32-bit words (split_words)
+void split_constants(const Plan& p, int words, SplitMod* out);
 
 // CRT table: Sum_t r_t W_t - q M on 16-bit limbs, q from the sum's top two limbs in FP32 (the
 // reference estimates q from the residues in FP32, src/ozaki2_gpu.hpp:526-588)
