@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(256, CPLX ? 2 : (L <= 8 ? 4 : 3)) crt_kernel(c
         if (P.items[mid].block0 <= static_cast<int64_t>(blockIdx.x)) lo = mid;
         else hi = mid - 1;
     }
-    const CrtItem* __restrict__ I = P.items + lo;
+    const CrtItem* I = P.items + lo;
     int64_t jblk, ib;
     divmod_index(static_cast<int64_t>(blockIdx.x) - I->block0, I->iblocks, jblk, ib);
     const int tk = I->tk, s = P.s;
@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(256, CPLX ? 2 : (L <= 8 ? 4 : 3)) crt_kernel(c
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    auto column_max = [&](int64_t j) { return j + (lane & (COLS - 1)) < n ? __ldg(maxB + j + (lane & (COLS - 1))) : 0ull; };
+    auto column_max = [&](int64_t j) { return j + (lane & (COLS - 1)) < n ? maxB[j + (lane & (COLS - 1))] : 0ull; };
     unsigned long long mb = 0;
     if (j0 < jend) {
         fetch(0, j0);

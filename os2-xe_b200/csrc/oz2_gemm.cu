@@ -134,7 +134,7 @@ __device__ __forceinline__ void decode(const GemmParams& P, int64_t job, Job& J)
         if (P.items[mid].job0 <= job) lo = mid;
         else hi = mid - 1;
     }
-    const GemmItem* __restrict__ I = P.items + lo;
+    const GemmItem* I = P.items + lo;
     // 32-bit arithmetic: an item's jobs (groups * s * tiles) are bounded by its residue planes,
     // s m n bytes of device memory, so they stay far below 2^32
     const uint32_t local = static_cast<uint32_t>(job - I->job0), tiles = static_cast<uint32_t>(I->tiles);
@@ -437,7 +437,7 @@ __global__ void __launch_bounds__(gemm_threads<KIND>(), 1) gemm_i8_modm_kernel(c
 #pragma unroll
                             for (int b = 0; b < 32; ++b) {
                                 const int64_t i = i0 + b;
-                                const float ri = i < mm ? static_cast<float>(__ldg(J.I->cert_ra + i)) : 0.0f;
+                                const float ri = i < mm ? static_cast<float>(J.I->cert_ra[i]) : 0.0f;
                                 if (ri > 0.0f) {
                                     const float g = __uint_as_float(cur[b]);
                                     if (g > 0.0f) {
@@ -564,7 +564,7 @@ __global__ void __launch_bounds__(gemm_threads<KIND>(), 1) gemm_i8_modm_kernel(c
                 // i of this warp's half, four entries per word, eight words per pass
                 if (ok) {
                     dev::tmem_store_wait();
-                    const GemmItem* __restrict__ I = J.I;
+                    const GemmItem* I = J.I;
                     const int tk = I->crt_tk, s_ = I->s;
                     const int64_t j = static_cast<int64_t>(J.tj) * kGemmJ + quarter * 32 + lane;
                     const int64_t mm = I->m, nn = I->n;

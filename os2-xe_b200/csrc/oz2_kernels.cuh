@@ -168,8 +168,12 @@ int64_t crt_item_blocks(CrtItem& it, int64_t block0);
 // A launch that may start while the kernel before it on the stream still runs: its blocks are placed as that
 // one's drain and wait in dev::chain_wait(), so the launch latency and the prologue are hidden. Only for kernels
 // that call chain_wait() in every block before their first global access; the completion of each then implies
-// the completion of all before it, so a later plain launch, copy or event sees them all. Back to back, with the
-// shared launches: 128^3 38 -> 20 us per call, 1024^3 76 -> 56; 6000 x 6000 x 384 578 -> 570.
+// the completion of all before it, so a later plain launch, copy or event sees them all. What the kernels before it
+// write (item tables, row maxima, planes) may change while such a kernel is already resident: it is read by ordinary
+// loads, copies or atomics, never through const __restrict__ or __ldg, which promise that it is constant for as long
+// as the kernel lives and may be moved above chain_wait(). The caller's operands are constant for that long: every
+// call's first launch is plain. Back to back, with the shared launches: 128^3 38 -> 20 us per call, 1024^3 76 -> 56;
+// 6000 x 6000 x 384 578 -> 570.
 template <class... P, class... A>
 void launch_chained(void (*kernel)(P...), unsigned grid, unsigned threads, size_t smem, cudaStream_t st, A... args) {
     cudaLaunchAttribute at{};

@@ -45,7 +45,7 @@ __device__ __forceinline__ int find_item(const Item* items, int count, int64_t b
 // Otherwise: inner index contiguous, one warp per row and a k range per block.
 // The layout is the item's, so both operands share one launch.
 template <bool CPLX>
-__global__ void __launch_bounds__(256) scale_kernel(const ScaleItem* __restrict__ items, int count) {
+__global__ void __launch_bounds__(256) scale_kernel(const ScaleItem* items, int count) {
     dev::chain_wait();
     dev::chain_next();
     const ScaleItem* I = items + find_item(items, count, blockIdx.x);
@@ -293,7 +293,7 @@ struct SplitShared {
     uint4 c[kMaxModuliExt / 4][4];
 };
 template <int NW>
-__device__ __forceinline__ void split_consts(const SplitItem* __restrict__ I, SplitShared<NW>& S) {
+__device__ __forceinline__ void split_consts(const SplitItem* I, SplitShared<NW>& S) {
     const int lane = static_cast<int>(threadIdx.x & 31), g = lane >> 2, c = lane & 3, nmod = I->s;
     for (int grp = static_cast<int>(threadIdx.x >> 5); 4 * grp < nmod; grp += kSplitThreads / 32) {
         const int t = 4 * grp + (g & 3);
@@ -337,7 +337,7 @@ struct SplitFetch {
     uint32_t dst;     // its shared-memory address in tile 0
     int64_t step;     // source bytes between the thread's rows (k contiguous) or inner indices
 
-    __device__ __forceinline__ SplitFetch(const SplitItem* __restrict__ I, uint32_t tile0, int64_t r0, int kb0) {
+    __device__ __forceinline__ SplitFetch(const SplitItem* I, uint32_t tile0, int64_t r0, int kb0) {
         const int tid = static_cast<int>(threadIdx.x), lane = tid & 31;
         const int64_t ldx = I->ldx, k0 = static_cast<int64_t>(kb0) * kTileK;
         int r, p;
@@ -395,7 +395,7 @@ struct SplitFetch {
     }
 
     // the tile at k0, with every access checked
-    __device__ __noinline__ static void edge(const SplitItem* __restrict__ I, uint32_t tile, int64_t r0, int k0) {
+    __device__ __noinline__ static void edge(const SplitItem* I, uint32_t tile, int64_t r0, int k0) {
         const int64_t rows = I->rows - r0, ldx = I->ldx;
         const int k = static_cast<int>(I->k) - k0;
         const char* X = reinterpret_cast<const char*>(I->X);
@@ -416,7 +416,7 @@ struct SplitFetch {
 // below I->rows (the GEMM never uses a padding row's products) and of all inner indices (zero past
 // k). mx[r - mbase]: the rows' maximum bits. The next tile's copies run under this one's work.
 template <int NW, bool CPLX, bool ROWC>
-__device__ __forceinline__ void split_tiles(const SplitItem* __restrict__ I, SplitShared<NW>& S, int64_t r0, int kb0,
+__device__ __forceinline__ void split_tiles(const SplitItem* I, SplitShared<NW>& S, int64_t r0, int kb0,
                                             int kb1, const unsigned long long* mx, int64_t mbase) {
     constexpr int R = split_rows<CPLX>() / 8, NG = CPLX ? 2 : 1, NP = CPLX ? 3 : 1, E = CPLX ? 16 : 8;
     const int lane = static_cast<int>(threadIdx.x & 31), w8 = static_cast<int>(threadIdx.x >> 5);
@@ -534,12 +534,12 @@ __device__ __forceinline__ void split_tiles(const SplitItem* __restrict__ I, Spl
 // (one branch per block), so both operands share one launch.
 template <int NW, bool CPLX>
 __global__ void __launch_bounds__(kSplitThreads, CPLX || NW == 2 ? 2 : 3)
-    split_kernel(const SplitItem* __restrict__ items, int count) {
+    split_kernel(const SplitItem* items, int count) {
     __shared__ SplitShared<NW> S;
     // no chain_next: GEMM blocks placed while these drain land on the SMs in the order they fall free, and tiles
     // that share operands drift apart (8192^3, s = 14: 7.75 ms, 8.3 ms so placed)
     dev::chain_wait();
-    const SplitItem* __restrict__ I = items + find_item(items, count, blockIdx.x);
+    const SplitItem* I = items + find_item(items, count, blockIdx.x);
     const int64_t local = static_cast<int64_t>(blockIdx.x) - I->block0;
     int64_t bx, by;
     divmod_index(local, I->rblocks, by, bx);

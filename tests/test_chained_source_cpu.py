@@ -1,0 +1,47 @@
+"""The rule of chained launches, checked on the sources: a kernel that may be resident while the kernels before
+it still write its item tables, row maxima and planes calls chain_wait() and promises nothing constant about that data
+(no __restrict__; __ldg only on the caller's operands, which are constant from a call's first launch on)."""
+import os
+import re
+
+import pytest
+
+SRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "os2-xe_b200", "csrc")
+FILES = {f: open(os.path.join(SRC, f)).read() for f in os.listdir(SRC) if f.endswith((".cu", ".cuh"))}
+CHAINED = sorted({(f, k) for f, text in FILES.items() for k in re.findall(r"launch_chained\((\w+)\s*<", text)})
+# functions of the chained kernels that read their items
+HELPERS = [("oz2_split.cu", h) for h in ("find_item", "split_consts", "SplitFetch", "edge", "split_tiles")] + [("oz2_gemm.cu", "decode")]
+OPERANDS = {"scale_kernel": {"X", "row"}}  # pointers into op(A), op(B) read through __ldg
+
+
+def body(text, name):
+    """the definition of `name`, from its parameter list to its closing brace"""
+    for m in re.finditer(r"\b%s\(" % name, text):
+        depth, i = 0, m.end() - 1
+        while True:  # past the parameter list
+            depth += {"(": 1, ")": -1}.get(text[i], 0)
+            i += 1
+            if depth == 0:
+                break
+        if not re.match(r"\s*\{", text[i:]):
+            continue  # a call or a declaration
+        while True:
+            depth += {"{": 1, "}": -1}.get(text[i], 0)
+            i += 1
+            if depth == 0 and text[i - 1] == "}":
+                return text[m.start():i]
+    raise AssertionError(name)
+
+
+def test_the_chained_kernels_are_found():
+    assert {k for _, k in CHAINED} == {"scale_kernel", "split_kernel", "gemm_i8_modm_kernel", "crt_kernel"}
+
+
+@pytest.mark.parametrize("where,name", CHAINED + HELPERS)
+def test_no_constant_promise(where, name):
+    text = body(FILES[where], name)
+    if (where, name) in CHAINED:
+        assert "dev::chain_wait();" in text
+    assert "__restrict__" not in text
+    for arg in re.findall(r"__ldg\((\w+)", text):
+        assert arg in OPERANDS.get(name, ()), arg
