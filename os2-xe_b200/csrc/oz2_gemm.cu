@@ -231,7 +231,10 @@ __global__ void __launch_bounds__(gemm_threads<KIND>(), 1) gemm_i8_modm_kernel(c
                 int w = 1;
                 if (!whole || lane == 0)
                     w = dev::mbar_wait(jobs_full(b), (n / (2 * kJobBatch)) & 1u, abort_flag, P.err, dev::kErrTimeoutJobs, P.wait_ns);
-                if (whole) w = __shfl_sync(0xFFFFFFFFu, w, 0);
+                if (whole) {
+                    w = __shfl_sync(0xFFFFFFFFu, w, 0);
+                    __syncwarp();  // orders the other lanes' reads after lane 0's wait; a shuffle orders no memory
+                }
                 if (!w) {
                     ok = false;
                     return false;
@@ -259,6 +262,7 @@ __global__ void __launch_bounds__(gemm_threads<KIND>(), 1) gemm_i8_modm_kernel(c
             if (lane == 0)
                 w = dev::mbar_wait(jobs_empty(b & 1), ((b >> 1) & 1u) ^ 1u, abort_flag, P.err, dev::kErrTimeoutJobs, P.wait_ns);
             if (!__shfl_sync(0xFFFFFFFFu, w, 0)) break;
+            __syncwarp();  // the batch's last readers before this warp's writes
             const int64_t job = blockIdx.x + (static_cast<int64_t>(b) * kJobBatch + lane) * nprog;
             Job& J = job_ring[(b & 1) * kJobBatch + lane];
             if (job < P.jobs) decode<BN, KIND>(P, job, J);

@@ -1,6 +1,7 @@
-"""The rule of chained launches, checked on the sources: a kernel that may be resident while the kernels before
+"""Rules of memory order, checked on the sources. Chained launches: a kernel that may be resident while the kernels before
 it still write its item tables, row maxima and planes calls chain_wait() and promises nothing constant about that data
-(no __restrict__; __ldg only on the caller's operands, which are constant from a call's first launch on)."""
+(no __restrict__; __ldg only on the caller's operands, which are constant from a call's first launch on). The GEMM's job ring: a
+warp whose lane 0 waited on an mbarrier touches the ring after __syncwarp(), as a shuffle orders no memory."""
 import os
 import re
 
@@ -45,3 +46,12 @@ def test_no_constant_promise(where, name):
     assert "__restrict__" not in text
     for arg in re.findall(r"__ldg\((\w+)", text):
         assert arg in OPERANDS.get(name, ()), arg
+
+
+def test_job_ring_is_ordered():
+    text = body(FILES["oz2_gemm.cu"], "gemm_i8_modm_kernel")
+    waits = [m.end() for m in re.finditer(r"mbar_wait\(jobs_(?:full|empty)\(", text)]
+    assert len(waits) == 2
+    for at in waits:
+        use = text.index("job_ring[", at)
+        assert "__syncwarp();" in text[at:use]
