@@ -140,7 +140,7 @@ __device__ __forceinline__ void decode(const GemmParams& P, int64_t job, Job& J)
     const uint32_t local = static_cast<uint32_t>(job - I->job0), tiles = static_cast<uint32_t>(I->tiles);
     const uint32_t gt = CRTF ? 0u : local / tiles, tile = local - gt * tiles;
     const uint32_t tiles_i = static_cast<uint32_t>(I->tiles_i), tiles_j = static_cast<uint32_t>(I->tiles_j);
-    const uint32_t group_j = static_cast<uint32_t>(P.group_j), per_grp = group_j * tiles_i;
+    const uint32_t group_j = min(static_cast<uint32_t>(P.group_j), tiles_j), per_grp = group_j * tiles_i;  // at most `tiles`
     const uint32_t grp = tile / per_grp, rem = tile - grp * per_grp;
     const uint32_t first_j = grp * group_j, gj = min(group_j, tiles_j - first_j), qj = rem / gj;
     const int tj = static_cast<int>(first_j + (rem - qj * gj)), ti = static_cast<int>(qj);
