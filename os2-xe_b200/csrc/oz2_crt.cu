@@ -175,7 +175,8 @@ __global__ void __launch_bounds__(256, CPLX ? 2 : (L <= 8 ? 4 : 3)) crt_kernel(c
                         asm volatile("ld.shared.u32 %0, [%1];"
                                      : "=r"(w[u])
                                      : "r"((COLS == 4 ? slot : slot ^ ((((u & 1) << 1) ^ c) << 5)) + (h * PL + 16 * x) * (32 * COLS) +
-                                           (COLS == 4 ? u * 128 : (u >> 1) * 128)));
+                                           (COLS == 4 ? u * 128 : (u >> 1) * 128))
+                                     : "memory");
                     transpose4(w[0], w[1], w[2], w[3], o[h][x]);
                 }
             auto limbs = [&](auto sg) {

@@ -449,8 +449,9 @@ __device__ __forceinline__ void split_tiles(const SplitItem* I, SplitShared<NW>&
         if (e != e1) odd |= 1u << u;
     }
     const double im_sign = CPLX && I->conj ? -1.0 : 1.0;  // residues of -y are the negated residues of y
-    // shared-memory address of the lane's element j = 0 of the warp's first row
-    const uint32_t el0 = tile0 + split_slot<CPLX, ROWC>(R * w8, 16 * ch + sub) * E;
+    const unsigned char* tiles = reinterpret_cast<const unsigned char*>(&S.tile);
+    // byte in a tile of the lane's element j = 0 of the warp's first row
+    const uint32_t el0 = split_slot<CPLX, ROWC>(R * w8, 16 * ch + sub) * E;
     // as a receiver: modulus g % 4 of each group of four, 16-byte chunk 2 c + g / 4 of the row
     const int g = n, c = q, tl = g & 3, nmod = I->s;
     const int64_t plane_bytes = I->plane_bytes, gstride = nmod * plane_bytes, tstep = 4 * plane_bytes;
@@ -474,8 +475,12 @@ __device__ __forceinline__ void split_tiles(const SplitItem* I, SplitShared<NW>&
                                                 : (CPLX ? (el0 ^ ((j & 1) << 6)) + ((j & 2) << 6) : (el0 ^ (j << 5))) +
                                                       u * (kTileK * E));
                 double y[NG];
-                if (CPLX) asm("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(y[0]), "=d"(y[NG - 1]) : "r"(at));
-                else asm("ld.shared.f64 %0, [%1];" : "=d"(y[0]) : "r"(at));
+                if constexpr (CPLX) {  // ordinary loads: the copies' waits above order them
+                    const double2 v = *reinterpret_cast<const double2*>(tiles + at);
+                    y[0] = v.x, y[1] = v.y;
+                } else {
+                    y[0] = *reinterpret_cast<const double*>(tiles + at);
+                }
 #pragma unroll
                 for (int h = 0; h < NG; ++h) {
                     double x = y[h] * s1[u];

@@ -1,7 +1,9 @@
 """Rules of memory order, checked on the sources. Chained launches: a kernel that may be resident while the kernels before
 it still write its item tables, row maxima and planes calls chain_wait() and promises nothing constant about that data
 (no __restrict__; __ldg only on the caller's operands, which are constant from a call's first launch on). The GEMM's job ring: a
-warp whose lane 0 waited on an mbarrier touches the ring after __syncwarp(), as a shuffle orders no memory."""
+warp whose lane 0 waited on an mbarrier touches the ring after __syncwarp(), as a shuffle orders no memory. Inline assembly: what
+reads or writes memory, or waits for it, is volatile and clobbers memory (a load without them is a function of its address
+to the compiler, which may keep its value over a refill)."""
 import os
 import re
 
@@ -55,3 +57,24 @@ def test_job_ring_is_ordered():
     for at in waits:
         use = text.index("job_ring[", at)
         assert "__syncwarp();" in text[at:use]
+
+
+def asm_statements(text):
+    for m in re.finditer(r"\basm\s*(volatile)?\s*\(", text):
+        depth, i, quoted = 1, m.end(), False
+        while depth:
+            c = text[i]
+            if c == '"':
+                quoted = not quoted
+            elif not quoted:
+                depth += {"(": 1, ")": -1}.get(c, 0)
+            i += 1
+        yield m.group(1), text[m.end():i]
+
+
+@pytest.mark.parametrize("where", sorted(FILES))
+def test_assembly_that_touches_memory(where):
+    for volatile, stmt in asm_statements(FILES[where]):
+        code = " ".join(re.findall(r'"((?:[^"\\]|\\.)*)"', stmt.split('"=')[0]))
+        if re.search(r"\b(ld|st|atom|red|cp)\.|mbarrier|tcgen05|fence|griddepcontrol", code):
+            assert volatile and '"memory"' in stmt, code
