@@ -35,7 +35,8 @@ namespace {
 // had to be moved to registers), then DRAM. Four blocks per SM up to 8 limbs (64 registers), three
 // above, two for complex operands. CRT stage, start -> now, alternating in one process: 8192^2, s = 16,
 // beta != 0 1019 -> 595 us (332 us of DRAM time at the measured copy rate); 6144^2, s = 20 757 -> 566;
-// 4096^2, s = 24 315 -> 193, s = 32 (a tcgen05 form before) 451 -> 221; ZGEMM 4096^2, s = 16 720 -> 429;
+// 4096^2, s = 24 315 -> 193, s = 32 (a tcgen05 form before) 451 -> 221; ZGEMM 4096^2, s = 16 720 -> 429, s = 18
+// 890 -> 482 (736 with one block per SM, before complex plans kept 24 planes only), 1000^2, s = 18 60 -> 56 (87);
 // 512 grouped problems 1506 -> 1111.
 // columns of a warp tile: a 128-byte line per plane, or half of one where shared memory would cost blocks
 constexpr int crt_cols(int L, bool cplx) { return cplx || L > 8 ? 2 : 4; }
@@ -44,7 +45,9 @@ template <int L, bool CPLX>
 struct alignas(128) CrtWarp {  // a warp's shared memory
     static constexpr int KH = L <= 8 ? 1 : 2, G = CPLX ? 3 : 1, W = CPLX ? 2 : 1;
     static constexpr int kCols = crt_cols(L, CPLX);
-    uint8_t res[2][G][16 * KH][32 * kCols];
+    // residue planes kept: complex plans stop at 24 moduli, and with 32 planes a second block would not fit the SM
+    static constexpr int kPlanes = KH == 1 ? 16 : (CPLX ? kMaxModuli : kMaxModuliExt);
+    uint8_t res[2][G][kPlanes][32 * kCols];
     uint32_t limb[W][32][crt_pitch(L)];
 };
 struct CrtParams {
@@ -80,10 +83,11 @@ __device__ __forceinline__ void mma_res_k32(uint32_t (&d)[4], uint32_t a0, uint3
             : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0));
 }
 
+constexpr int crt_blocks(int L, bool cplx) { return cplx ? 2 : (L <= 8 ? 4 : 3); }  // per SM
 template <int L, bool CPLX>
-__global__ void __launch_bounds__(256, CPLX ? 2 : (L <= 8 ? 4 : 3)) crt_kernel(const __grid_constant__ CrtParams P) {
+__global__ void __launch_bounds__(256, crt_blocks(L, CPLX)) crt_kernel(const __grid_constant__ CrtParams P) {
     using Warp = CrtWarp<L, CPLX>;
-    constexpr int KH = Warp::KH, G = Warp::G, NT = (L + 3) / 4, PL = 16 * KH, COLS = Warp::kCols, W2 = Warp::W;
+    constexpr int KH = Warp::KH, G = Warp::G, NT = (L + 3) / 4, PL = Warp::kPlanes, COLS = Warp::kCols, W2 = Warp::W;
     extern __shared__ __align__(128) uint8_t smem_raw[];
     const int warp = static_cast<int>(threadIdx.x >> 5), lane = static_cast<int>(threadIdx.x & 31);
     Warp& S = reinterpret_cast<Warp*>(smem_raw)[warp];
@@ -145,7 +149,9 @@ __global__ void __launch_bounds__(256, CPLX ? 2 : (L <= 8 ? 4 : 3)) crt_kernel(c
         fetch(0, j0);
         mb = column_max(j0);
     }
-    // the lane's words of a column: moduli 4 c + u, rows g + 8 e
+    // the lane's words of a column: moduli 4 c + u, and 16 + 4 c + u (past the kept planes any word will do: its
+    // weights are zero), rows g + 8 e
+    const uint32_t upper = 16 + 4 * c < PL ? 16 * (32 * COLS) : 0;
     const uint32_t at = dev::smem_addr(&S.res[0][0][0][0]) + 4 * c * (32 * COLS) + 4 * g;
     for (int buf = 0; j0 < jend; j0 += jstep, buf ^= 1) {
         const int Ec = unscale_exponent(mb, tk);  // of column j0 + lane % COLS
@@ -174,8 +180,8 @@ __global__ void __launch_bounds__(256, CPLX ? 2 : (L <= 8 ? 4 : 3)) crt_kernel(c
                     for (int u = 0; u < 4; ++u)
                         asm volatile("ld.shared.u32 %0, [%1];"
                                      : "=r"(w[u])
-                                     : "r"((COLS == 4 ? slot : slot ^ ((((u & 1) << 1) ^ c) << 5)) + (h * PL + 16 * x) * (32 * COLS) +
-                                           (COLS == 4 ? u * 128 : (u >> 1) * 128))
+                                     : "r"((COLS == 4 ? slot : slot ^ ((((u & 1) << 1) ^ c) << 5)) + h * PL * (32 * COLS) +
+                                           x * upper + (COLS == 4 ? u * 128 : (u >> 1) * 128))
                                      : "memory");
                     transpose4(w[0], w[1], w[2], w[3], o[h][x]);
                 }
@@ -250,7 +256,12 @@ __global__ void __launch_bounds__(256, CPLX ? 2 : (L <= 8 ? 4 : 3)) crt_kernel(c
 }
 
 template <int L, bool CPLX>
-constexpr int crt_smem() { return 8 * static_cast<int>(sizeof(CrtWarp<L, CPLX>)); }
+constexpr int crt_smem() {
+    constexpr int bytes = 8 * static_cast<int>(sizeof(CrtWarp<L, CPLX>));
+    // the blocks that the registers are cut for have room in an SM's 228 KB (1 KB of it reserved per block)
+    static_assert(crt_blocks(L, CPLX) * (bytes + 1024) <= 228 * 1024, "CRT blocks per SM");
+    return bytes;
+}
 
 // by the plan's limbs; complex CRTs stop at s = 24 (zgemm is the reference's call): 12 limbs
 template <int L>
