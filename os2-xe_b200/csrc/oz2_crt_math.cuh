@@ -4,8 +4,8 @@
 // x = Sum_t r_t W_t - q M with q the nearest integer to Sum_t r_t W_t / M (|x| <= M/4), rounded once
 // to double. Everything runs on 16-bit limbs: a_l = Sum_t r_t W_t[l] (|r_t| <= 255, so
 // below 32 * 255 * 2^16 < 2^29), then
-//   q      from the top two limbs of the sum in FP32: the limbs below add less than 0.05 to Sum / M
-//          (0.03 for complex operands' combined sums), so the estimate errs by less than 1/4;
+//   q      from the top two limbs of the sum in FP32: the limbs below add at most 0.05 to Sum / M
+//          (0.03 for complex operands' combined sums; the plan's build checks both), so the estimate errs by less than 1/4;
 //   limbs  c_l = a_l - q M_l + (c_{l-1} >> 16), one multiply-add and one shifted add each: the low 16
 //          bits of c_0 .. c_{L-2} and all of c_{L-1} are x in two's complement;
 //   RNE    the three top 32-bit words h, m, l as doubles (l with a sticky bit for the words below):

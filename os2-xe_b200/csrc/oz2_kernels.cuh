@@ -148,7 +148,7 @@ struct CrtItem {
 int64_t scale_item_blocks(ScaleItem& it, int num_sms, int64_t block0);
 int64_t slice_item_blocks(SplitItem& it, int64_t block0);
 // the split's geometry for the kernel that will run the item: the tensor-core split for real
-// items while it is selected, else split_item_blocks; sets it.tc
+// items while it is selected, else rows by k spans of split_launch_shape; sets it.tc
 int64_t split_geometry(SplitItem& it, int64_t block0);
 // the k blocks per block of a split launch's items, before split_geometry
 void split_launch_shape(SplitItem* items, int count);

@@ -136,13 +136,14 @@ struct Templates {
             p.y[t] = static_cast<uint32_t>(y);
         }
         std::memcpy(p.M, M.w, sizeof M.w);
-        // what the CRT's quotient leaves out, the limbs of Sum r_t W_t below the top two: under 0.1 M (two
-        // such sums for complex operands, s <= 24), inside the 1/4 that |x| <= M/4 leaves
+        // what the CRT's quotient leaves out, the limbs of Sum r_t W_t below the top two: at most 0.05 M (s = 32 has
+        // 0.0475), and 0.015 M for the sets complex operands use (s = 23: 0.0118), whose combined sums leave out twice
+        // that; inside the 1/4 that |x| <= M/4 leaves
         double rest = 0.0;
         for (int t = 0; t < s; ++t)
             for (int l = 0; l < limbs16_for(s) - 2; ++l)
                 rest += 255.0 * std::exp2(16.0 * l - p.log2M) * ((p.W[t][l / 2] >> (16 * (l & 1))) & 0xFFFFu);
-        if (rest > 0.1) return 3;
+        if (rest > (s <= kMaxModuli ? 0.015 : 0.05)) return 3;
         mod_constants(p, p.mc);
         return 0;
     }
