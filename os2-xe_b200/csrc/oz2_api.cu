@@ -375,7 +375,7 @@ int64_t split_geom(SplitItem& it, int64_t b0) { return split_geometry(it, b0); }
 int64_t crt_geom(CrtItem& it, int64_t b0) { return crt_item_blocks(it, b0); }
 
 // Appends split, GEMM and CRT operations for a list of tasks (launches grouped by kernel variant)
-void plan_tasks(Program& prog, const std::vector<Task>& tasks, const GemmConfig& cfg) {
+void plan_tasks(Program& prog, const std::vector<Task>& tasks, const GemmConfig& cfg, int num_sms) {
     // split: group by (complex / fused scale, limb path: narrow, wide, widest), and by layout where the kernel
     // is one layout's (the fused and the tensor-core split); 128^3: one launch 6 us, one per layout 11 us
     std::map<std::tuple<int, int, int>, std::vector<SplitItem>> split_groups;
@@ -397,7 +397,7 @@ void plan_tasks(Program& prog, const std::vector<Task>& tasks, const GemmConfig&
             add_split(it, wide);
         }
     }
-    for (auto& kv : split_groups) split_launch_shape(kv.second.data(), static_cast<int>(kv.second.size()));
+    for (auto& kv : split_groups) split_launch_shape(kv.second.data(), static_cast<int>(kv.second.size()), num_sms);
     for (auto& kv : split_groups) add_grouped(prog, kv.second, Op::Split, split_geom, nullptr, false);
     Op mk;
     mk.kind = Op::Mark;
@@ -523,7 +523,7 @@ void plan_tasks(Program& prog, const std::vector<Task>& tasks, const GemmConfig&
     }
     for (auto& kv : crt_groups)
         crt_launch_shape(kv.second.second.data(), static_cast<int>(kv.second.second.size()), *kv.second.first,
-                         kv.first.second != 0);
+                         kv.first.second != 0, num_sms);
     for (auto& kv : crt_groups)
         add_grouped(prog, kv.second.second, Op::Crt, crt_geom, kv.second.first, kv.first.second != 0);
     mk.stage = kCrt;
@@ -868,7 +868,7 @@ int run_single(oz2_context* h, const Prob& p) {
         for (int64_t i0 = 0; i0 < p.m; i0 += L.mb) {
             Task t{&p, i0, j0, std::min(L.mb, p.m - i0), std::min(L.nb, p.n - j0), L.pm > 1 || j0 == 0, i0 == 0,
                    maxA, maxB, planesA, planesB, resid, ldr, fa, fb};
-            plan_tasks(prog, {t}, cfg);
+            plan_tasks(prog, {t}, cfg, h->num_sms);
         }
     }
     if (prog.blob.size() > align256(desc_bytes_single(L.pm, L.pn)) || (first && prog.blob.size() > kScaleFirstBytes))
@@ -957,7 +957,7 @@ int run_grouped(oz2_context* h, std::vector<Prob>& probs) {
         ms.bytes = max_end;
         prog.ops.push_back(ms);
         plan_scale(h, prog, sc);
-        plan_tasks(prog, tasks, cfg);
+        plan_tasks(prog, tasks, cfg, h->num_sms);
         if (static_cast<size_t>(dev_desc - h->ws) + prog.blob.size() > h->ws_size)
             return fail(h, OZ2_EINTERNAL, "oz2: descriptor region too small");
         if ((st = check_grid(h, prog))) return st;
@@ -1773,7 +1773,7 @@ int run_adaptive(oz2_context* h, std::vector<Prob>& base, const std::vector<int>
             const GemmConfig cfg = config_for(h, bp);
             h->last_cfg = cfg;
             Program prog;
-            plan_tasks(prog, tasks, cfg);
+            plan_tasks(prog, tasks, cfg, h->num_sms);
             if (obase_desc + prog.blob.size() > h->ws2_size)
                 return fail(h, OZ2_EINTERNAL, "oz2: descriptor region too small");
             if ((st2 = check_grid(h, prog))) return st2;

@@ -416,13 +416,13 @@ __global__ void __launch_bounds__(256) oz1_horner_kernel(const int64_t* __restri
 
 }  // namespace
 
-void crt_launch_shape(CrtItem* items, int count, const Plan& plan, bool cplx) {
+void crt_launch_shape(CrtItem* items, int count, const Plan& plan, bool cplx, int num_sms) {
     // a block and turn: 32 rows by 8 warps' columns; up to 8 turns per block while about eight blocks per
     // SM remain in the launch
     const int L = limbs16_for(plan.s), cols = 8 * crt_cols(L, cplx);
     int64_t turns = 0;
     for (int q = 0; q < count; ++q) turns += ceil_div(items[q].m, 32) * ceil_div(items[q].n, cols);
-    const int jc = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(8, turns / (8 * 148))));
+    const int jc = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(8, turns / (8 * num_sms))));
     for (int q = 0; q < count; ++q) {
         items[q].cols = cols;
         items[q].jc = jc;

@@ -151,7 +151,7 @@ int64_t slice_item_blocks(SplitItem& it, int64_t block0);
 // items while it is selected, else rows by k spans of split_launch_shape; sets it.tc
 int64_t split_geometry(SplitItem& it, int64_t block0);
 // the k blocks per block of a split launch's items, before split_geometry
-void split_launch_shape(SplitItem* items, int count);
+void split_launch_shape(SplitItem* items, int count, int num_sms);
 // process-wide selection of the real split: 0 the mma.sync kernel (default), 1 the tcgen05 split
 void set_split_path(int tc);
 int split_path();
@@ -162,7 +162,7 @@ int split_path();
 void set_scale_fusion(int on);
 bool fuse_scale(bool cplx, bool row_contig, int64_t k);
 // sets the block shape of a CRT launch's items (all of one plan), before crt_item_blocks
-void crt_launch_shape(CrtItem* items, int count, const Plan& plan, bool cplx);
+void crt_launch_shape(CrtItem* items, int count, const Plan& plan, bool cplx, int num_sms);
 int64_t crt_item_blocks(CrtItem& it, int64_t block0);
 
 // A launch that may start while the kernel before it on the stream still runs: its blocks are placed as that

@@ -195,7 +195,7 @@ extern "C" int oz2_dgemm_noalloc(void* stream, char ta, char tb, int64_t m, int6
         sp.kb_total = gg.kb_total;
         sp.rows_pad = gg.rows_pad;
         for (int t = 0; t < s; ++t) sp.mc[t] = p.sm[t];
-        split_launch_shape(&sp, 1);
+        split_launch_shape(&sp, 1, num_sms);
         split_geometry(sp, 0);
     }
     GemmConfig cfg;
@@ -243,7 +243,7 @@ extern "C" int oz2_dgemm_noalloc(void* stream, char ta, char tb, int64_t m, int6
     c.ar = alpha;
     c.br = beta;
     c.C = C;
-    crt_launch_shape(&c, 1, p, false);
+    crt_launch_shape(&c, 1, p, false, num_sms);
     const int64_t crt_blocks = crt_item_blocks(c, 0);
     static_assert(sizeof(Tables) <= 8 * 1024, "item tables exceed their scratch region");
     unsigned char* dtab = scratch + o_D;

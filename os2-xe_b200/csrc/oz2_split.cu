@@ -1030,13 +1030,13 @@ int64_t slice_item_blocks(SplitItem& it, int64_t block0) {
     return it.rblocks * it.kblocks;
 }
 
-void split_launch_shape(SplitItem* items, int count) {
+void split_launch_shape(SplitItem* items, int count, int num_sms) {
     // up to 16 k blocks per block (a block's start costs about a tile's time: 8192^3 split 779, 697 and
     // 682 us with at most 3, 8 and 16) while about four blocks per SM remain in the launch
     int64_t tiles = 0;
     for (int q = 0; q < count; ++q)
         tiles += ceil_div(items[q].rows, items[q].cplx ? split_rows<true>() : split_rows<false>()) * items[q].kb_total;
-    const int span = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(16, tiles / (4 * 148))));
+    const int span = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(16, tiles / (4 * num_sms))));
     for (int q = 0; q < count; ++q) items[q].kspan = span;
 }
 
