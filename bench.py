@@ -202,7 +202,8 @@ def blas_threads():
 
 class CpuStream:
     """The reference's own CPU path (oracle/_ref: src/ozaki2_gpu.hpp built for the host, all host
-    threads; the C oracle where it was not built) over the stream's problems in stream order, each
+    threads; the C oracle where it was not built, reported as kind "port": that says nothing about the
+    reference's speed) over the stream's problems in stream order, each
     at its per-problem analytic s (the fixed s that meets the target). The reference's Ozaki2::gemm
     takes s <= 24 only (make_plan rejects more, src/ozaki2_gpu.hpp:160-161), so a problem whose
     analytic s is 25 runs as host FP64 DGEMM (numpy's BLAS, the reference bench's --cpu path,

@@ -33,7 +33,7 @@ namespace {
 // Bound: instruction issue (166 warp instructions per 32 entries at s = 16, 34 cycles of them the four
 // mma at 8.6 each; the dp2a form it replaces took 304, 72 of them two-cycle dot products whose weights
 // had to be moved to registers), then DRAM. Four blocks per SM up to 8 limbs (64 registers), three
-// above, two for complex operands. CRT stage, start -> now, alternating in one process: 8192^2, s = 16,
+// above, two for complex operands (of 24 residue planes above 8 limbs). CRT stage, start -> now, alternating in one process: 8192^2, s = 16,
 // beta != 0 1019 -> 595 us (332 us of DRAM time at the measured copy rate); 6144^2, s = 20 757 -> 566;
 // 4096^2, s = 24 315 -> 193, s = 32 (a tcgen05 form before) 451 -> 221; ZGEMM 4096^2, s = 16 720 -> 429, s = 18
 // 890 -> 482 (736 with one block per SM, before complex plans kept 24 planes only), 1000^2, s = 18 60 -> 56 (87);

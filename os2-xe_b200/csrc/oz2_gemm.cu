@@ -21,8 +21,9 @@
 //            kilobyte of the residue plane (layout in oz2_kernels.cuh)
 // Bound: at long k the tensor pipe under the power limit (4096^3: 80 % active at 1.6 of 1.97 GHz); a pair
 // of CTAs per tile (cta_group::2, a third less L2 traffic) measured 4-10 % slower. At few k-blocks the
-// epilogue: B200, 6000^2 x 384, s = 16, 305 -> 255 us and 512 grouped problems 2577 -> 2037 us with the
-// FP32 quotient and items found by a cursor instead of a search per job and role.
+// epilogue: B200, 6000^2 x 384, s = 16, 314 -> 249 us and 512 grouped problems 2553 -> 1444 us with the
+// FP32 quotient and, from eight jobs per CTA on, jobs decoded by a warp of their own (kKindQueue; the other kinds
+// search the item table once per job and role).
 // Every mbarrier wait is time-bounded; on expiry the kernel records an error code, drains its
 // in-flight copies and MMAs, frees TMEM and returns.
 #include <algorithm>
@@ -95,7 +96,9 @@ struct GemmParams {
 // k-blocks a job is shorter than the chain of item-table loads and divisions that finds it. B200, 4096^2 x
 // 256, s = 16: 161 -> 132 us; 512 grouped problems 2039 -> 1827. For launches of at least kQueueRounds jobs
 // per CTA: below, its first batch only adds latency (512^3 12.4 -> 14.5 us). At long k every role decodes
-// its own jobs (the extra warp measured 1.3 % slower there, 4096^2 x 2048 376 -> 382 us).
+// its own jobs (the extra warp measured 1.3 % slower there, 4096^2 x 2048 376 -> 382 us). One short item puts a
+// whole launch on this kernel; on mixed launches that costs nothing: 200 grouped problems of 256..4096, s = 16 / 20,
+// GEMM stage 24.5 / 30.5 ms, and 24.9 / 31.1 with every item on kKindResidue.
 constexpr int kKindResidue = 0, kKindOz1 = 1, kKindCert = 2, kKindCrt = 3, kKindShort = 4, kKindQueue = 5;
 constexpr int kQueueRounds = 8;
 template <int KIND>

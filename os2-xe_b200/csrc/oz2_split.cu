@@ -271,9 +271,11 @@ __device__ __forceinline__ void offset_words(double y, uint32_t (&W)[NW]) {
 // permute and 1/128 mma per lane (8.6 cycles of the scheduler per mma, measured) where dp4a took
 // two to four quarter-of-the-lanes dot products and a two-step quotient. The operand comes through
 // cp.async double buffering (rows contiguous: whole lines, transposed on the way out of shared
-// memory). Two blocks per SM of up to 128 registers on the narrow and complex paths, three of 80 on
-// the wider ones: more blocks with spilled or serialised accumulators measured slower. Stage times,
-// start -> now, alternating in one process: 8192^3 s = 16 1044 -> 682 us (498 us of DRAM time at the
+// memory). Two blocks per SM of up to 128 registers on the narrow and complex paths (three or four, with
+// spilled or serialised accumulators, measured slower), three of 80 on the wider ones, which spill 24 (three
+// words) and 72 bytes (four): against two blocks without spills 582 and 601 us at 6144^3 s = 20, 1574 and 1624
+// on 512 grouped problems, 269 and 275 at 4096^3 s = 24, but 149 and 130 at 4096^2 x 2048 s = 20 and 2.93
+// and 2.80 ms on 64 adaptive problems. Stage times, start -> now, alternating in one process: 8192^3 s = 16 1044 -> 682 us (498 us of DRAM time at the
 // measured copy rate), 6144^3 s = 20 (three words) 849 -> 575, 1024^2 x 262144 s = 16 3790 -> 2490,
 // ZGEMM 4096^3 s = 16 781 -> 424.
 constexpr int kSplitThreads = 256;
